@@ -1,6 +1,7 @@
 // Host side of the CUDA engine: compiles the operator algebra of a sweep
 // step into device work lists and drives the kernels of kernels.cu.
 #include "gpu_engine.h"
+#include "../../../include/bgpu.h"
 #include "k_dc.cuh"
 #include "k_noise.cuh"
 
@@ -489,9 +490,9 @@ void schedule_waves(const std::vector<double>& cost, int nblocks, std::vector<in
   }
 }
 
-void add_tasks(std::vector<dev::GemmTask>& t, int unit, int m, int n) {
-  for (int a = 0; a < (m + 63) / 64; ++a)
-    for (int b = 0; b < (n + 63) / 64; ++b) t.push_back({unit, a, b});
+void add_tasks(std::vector<dev::GemmTask>& t, int unit, int m, int n, int tile = dev::kGemmTile) {
+  for (int a = 0; a < (m + tile - 1) / tile; ++a)
+    for (int b = 0; b < (n + tile - 1) / tile; ++b) t.push_back({unit, a, b});
 }
 }  // namespace
 
@@ -719,8 +720,8 @@ void GpuEngine::plan_sigma(const Superblock& sb, SigmaPlan& plan) {
     });
   }
   laps.lap("stage-1 and items");
-  // stage 2: one unit per sector; a sector whose 64x64 tiles carry more K
-  // than a fair share of the FP64 pipe is split along its item list into
+  // stage 2: one unit per sector; a sector whose tiles carry more than a
+  // fair share of the FP64 pipe's work is split along its item list into
   // units writing partial sectors after the stage-1 intermediates, summed
   // into sigma in a fixed order by the build-copy kernel
   std::vector<dev::GemmUnit> u2;
@@ -728,22 +729,46 @@ void GpuEngine::plan_sigma(const Superblock& sb, SigmaPlan& plan) {
   std::vector<dev::GemmTask> t1, t2;
   std::vector<dev::CopyUnit> ru;
   std::vector<dev::CopyItem> ri;
-  double tile_k_total = 0.0;
+  // Work of a tile's share of a sector, in clocks of one SM: its FMAs at two
+  // a clock and about 150 clocks per item for the loads that no other block
+  // hides.  A block gets at least 1500 clocks (below that its own start, about
+  // 1 us, dominates) and at most a 32nd of an SM's share, so that uneven
+  // blocks level out (with a 16th the 16-orbital M=150 product took 3.4 ms
+  // and not 2.6; the former rule, a quarter of an SM's share and at least
+  // 4096 K, left the 20 sectors of 12 orbitals, M=50 to 20 blocks: 7.1 ms
+  // for the whole product, now 0.19).
+  auto tiles_of = [](const Superblock::Sector& S) {
+    return (double)((S.rows + dev::kGemmTile - 1) / dev::kGemmTile) * ((S.cols + dev::kGemmTile - 1) / dev::kGemmTile);
+  };
+  auto item_cost = [&](const Superblock::Sector& S, const dev::GemmItem& g) {
+    return 0.5 * S.rows * S.cols * g.k / tiles_of(S) + 150.0;
+  };
+  std::vector<double> tile_cost(sb.sectors.size(), 0.0);
+  double total_cost = 0.0;
   for (size_t s = 0; s < sb.sectors.size(); ++s) {
-    const auto& S = sb.sectors[s];
-    double k = 0.0;
-    for (auto& g : per_sector[s]) k += g.k;
-    tile_k_total += k * ((S.rows + 63) / 64) * ((S.cols + 63) / 64);
+    for (auto& g : per_sector[s]) tile_cost[s] += item_cost(sb.sectors[s], g);
+    total_cost += tile_cost[s] * tiles_of(sb.sectors[s]);
   }
-  const double tile_k_share = std::max(tile_k_total / (4.0 * sm_count()), 4096.0);
+  double share = std::max(total_cost / (32.0 * sm_count()), 1500.0);
+  auto chunks_of = [&](size_t s) {
+    return std::max(1, std::min((int)per_sector[s].size(), (int)std::ceil(tile_cost[s] / share)));
+  };
+  // the partial sectors stay within the fixed array of sigma_noalloc where the
+  // stage-1 intermediates leave room for them: one unit per sector needs none
+  if (scratch <= (int64_t)BGPU_NOALLOC_SCRATCH_DOUBLES)
+    for (;; share *= 1.5) {
+      int64_t extra = 0;
+      for (size_t s = 0; s < sb.sectors.size(); ++s) {
+        const int nc = chunks_of(s);
+        if (nc > 1) extra += (int64_t)nc * sb.sectors[s].rows * sb.sectors[s].cols;
+      }
+      if (extra == 0 || scratch + extra <= (int64_t)BGPU_NOALLOC_SCRATCH_DOUBLES) break;
+    }
   int64_t partial = scratch;  // partial sectors follow the stage-1 intermediates
   for (size_t s = 0; s < sb.sectors.size(); ++s) {
     const auto& S = sb.sectors[s];
     const auto& items = per_sector[s];
-    double k = 0.0;
-    for (auto& g : items) k += g.k;
-    const int ntiles = ((S.rows + 63) / 64) * ((S.cols + 63) / 64);
-    const int nchunks = std::max(1, std::min((int)items.size(), (int)std::ceil(k * ntiles / tile_k_share / ntiles)));
+    const int nchunks = chunks_of(s);
     if (nchunks <= 1) {
       dev::GemmUnit u{};
       u.c_buf = 3;
@@ -764,12 +789,12 @@ void GpuEngine::plan_sigma(const Superblock& sb, SigmaPlan& plan) {
     cu.m = S.rows;
     cu.n = S.cols;
     cu.ibeg = (int)ri.size();
-    const double per = k / nchunks;
+    const double per = tile_cost[s] / nchunks;
     size_t a = 0;
     for (int c = 0; c < nchunks && a < items.size(); ++c) {
       size_t e = a;
       double acc = 0.0;
-      while (e < items.size() && (acc < per || e == a || c == nchunks - 1)) acc += items[e++].k;
+      while (e < items.size() && (acc < per || e == a || c == nchunks - 1)) acc += item_cost(S, items[e++]);
       dev::GemmUnit u{};
       u.c_buf = 4;
       u.c_off = partial;
@@ -799,7 +824,9 @@ void GpuEngine::plan_sigma(const Superblock& sb, SigmaPlan& plan) {
   std::vector<std::pair<double, int>> cost;
   for (int u = 0; u < (int)u2.size(); ++u) {
     double c = 0;
-    for (int i = u2[u].ibeg; i < u2[u].iend; ++i) c += i2[i].k;
+    const int nth = (u2[u].m + dev::kGemmTile - 1) / dev::kGemmTile, ntw = (u2[u].n + dev::kGemmTile - 1) / dev::kGemmTile;
+    const double area = (double)u2[u].m * u2[u].n / (nth * ntw);
+    for (int i = u2[u].ibeg; i < u2[u].iend; ++i) c += 0.5 * area * i2[i].k + 150.0;
     cost.push_back({-c, u});
   }
   std::stable_sort(cost.begin(), cost.end());
@@ -855,7 +882,7 @@ void GpuEngine::plan_sigma(const Superblock& sb, SigmaPlan& plan) {
     du.push_back(u);
   }
   std::vector<dev::GemmTask> dtask;
-  for (int u = 0; u < (int)du.size(); ++u) add_tasks(dtask, u, du[u].rows, du[u].cols);
+  for (int u = 0; u < (int)du.size(); ++u) add_tasks(dtask, u, du[u].rows, du[u].cols, dev::kDiagTile);
   laps.lap("diagonal lists");
   plan.du.upload(du, stream_);
   plan.di.upload(di, stream_);
@@ -948,7 +975,7 @@ void GpuEngine::sigma_fp64(const Superblock& sb, const SigmaPlan& p, const doubl
   bufs.p[4] = scratch;
   cuda_check(dev::launch_gemm(bufs, p.u1.d, p.i1.d, p.t1.d, (int)p.t1.n, stream_), "sigma stage 1");
   cuda_check(dev::launch_gemm(bufs, p.u2.d, p.i2.d, p.t2.d, (int)p.t2.n, stream_), "sigma stage 2");
-  cuda_check(dev::launch_copy(bufs, out, p.ru.d, p.ri.d, (int)p.ru.n, stream_), "sigma stage-2 partial sums");
+  cuda_check(dev::launch_copy(bufs, out, p.ru.d, p.ri.d, (int)p.ru.n, stream_, 16), "sigma stage-2 partial sums");
   if (p.ecore != 0.0) cuda_check(dev::launch_axpy(p.ecore, psi, out, p.n, stream_), "ecore");
   sigma_flops += p.flops;
   ++sigma_calls;
@@ -2600,7 +2627,7 @@ void GpuEngine::sigma_timed(const Superblock& sb, const SigmaPlan& p, const doub
     cuda_check(dev::launch_gemm(bufs, p.u1.d, p.i1.d, p.t1.d, (int)p.t1.n, stream_), "sigma stage 1");
     cuda_check(cudaEventRecord(e[1], stream_), "record");
     cuda_check(dev::launch_gemm(bufs, p.u2.d, p.i2.d, p.t2.d, (int)p.t2.n, stream_), "sigma stage 2");
-    cuda_check(dev::launch_copy(bufs, out, p.ru.d, p.ri.d, (int)p.ru.n, stream_), "sigma stage-2 partial sums");
+    cuda_check(dev::launch_copy(bufs, out, p.ru.d, p.ri.d, (int)p.ru.n, stream_, 16), "sigma stage-2 partial sums");
     cuda_check(cudaEventRecord(e[2], stream_), "record");
     if (p.ecore != 0.0) cuda_check(dev::launch_axpy(p.ecore, psi, out, p.n, stream_), "ecore");
     cuda_check(cudaEventRecord(e[3], stream_), "record");

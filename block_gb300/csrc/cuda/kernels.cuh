@@ -45,6 +45,8 @@ struct GemmTask {
   int32_t unit;
   int32_t tm, tn;  // tile indices
 };
+constexpr int kGemmTile = 32;  // output-tile edge of the grouped GEMM
+constexpr int kDiagTile = 64;  // and of the diagonal tiles
 
 // dst rectangle (m x n at c_off, ldc) = sum of items [ibeg, iend)
 struct CopyUnit {
@@ -79,8 +81,9 @@ struct DiagItem {
 // launch helpers (return cudaGetLastError())
 cudaError_t launch_gemm(const Bufs& bufs, const GemmUnit* units, const GemmItem* items, const GemmTask* tasks,
                         int ntasks, cudaStream_t s);
+// split: blocks per unit
 cudaError_t launch_copy(const Bufs& bufs, double* dst, const CopyUnit* units, const CopyItem* items, int nunits,
-                        cudaStream_t s);
+                        cudaStream_t s, int split = 1);
 // d[off + i*cols + j] += sum over the unit's items, by 64 x 64 tiles of the
 // units (task.unit, task.tm, task.tn), the items as the K dimension of a GEMM
 cudaError_t launch_diag_tiles(const Bufs& bufs, double* d, const DiagUnit* units, const DiagItem* items,
