@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(256) tc_pack_kernel(TcBufs b, const TcPack* __
 }
 
 cudaError_t launch_tc_pack(const TcBufs& b, const TcPack* units, int nunits, cudaStream_t s) {
-  if (nunits > 0) tc_pack_kernel<<<dim3(nunits, 4), 256, 0, s>>>(b, units);
+  if (nunits > 0) tc_pack_kernel<<<dim3(nunits, pack_split(nunits)), 256, 0, s>>>(b, units);
   return cudaGetLastError();
 }
 
@@ -674,6 +674,9 @@ cudaError_t launch_tc_sigma_pairs(const TcBufs& b, const TcWork* work, const int
   return cudaGetLastError();
 }
 
+// Bound by the latency of the slot reads: few tiles (56 at 24 orbitals,
+// M=500) with tens of partials each, so every thread keeps eight reads in
+// flight and a 128 x 128 tile is spread over 32 blocks.
 __global__ void __launch_bounds__(256) tc_reduce_kernel(const float2* __restrict__ partials,
                                                          const TcTile* __restrict__ tiles,
                                                          const int64_t* __restrict__ slots, double* __restrict__ sigma) {
@@ -682,8 +685,18 @@ __global__ void __launch_bounds__(256) tc_reduce_kernel(const float2* __restrict
   for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < n; e += gridDim.y * blockDim.x) {
     double acc = 0.0;
     const int r = e / t.w, c = e % t.w;
-    for (int p = t.pbeg; p < t.pend; ++p) {
-      const float2 v = partials[slots[p] + (int64_t)r * t.pad + c];  // slots are h_a x h_b, row stride pad
+    const float2* src = partials + (int64_t)r * t.pad + c;  // slots are h_a x h_b, row stride pad
+    int p = t.pbeg;
+    // eight partials in flight per thread, summed in slot order
+    for (; p + 8 <= t.pend; p += 8) {
+      float2 v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = src[slots[p + i]];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc += (double)v[i].x + (double)v[i].y;
+    }
+    for (; p < t.pend; ++p) {
+      const float2 v = src[slots[p]];
       acc += (double)v.x + (double)v.y;
     }
     sigma[t.s_off + (int64_t)(t.r0 + r) * t.lds + t.c0 + c] = acc;
@@ -692,7 +705,7 @@ __global__ void __launch_bounds__(256) tc_reduce_kernel(const float2* __restrict
 
 cudaError_t launch_tc_reduce(const TcBufs& b, const TcTile* tiles, const int64_t* slots, int ntiles, double* sigma,
                              cudaStream_t s) {
-  if (ntiles > 0) tc_reduce_kernel<<<dim3(ntiles, 16), 256, 0, s>>>(b.partials, tiles, slots, sigma);
+  if (ntiles > 0) tc_reduce_kernel<<<dim3(ntiles, 32), 256, 0, s>>>(b.partials, tiles, slots, sigma);
   return cudaGetLastError();
 }
 

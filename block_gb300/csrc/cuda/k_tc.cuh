@@ -152,6 +152,11 @@ struct TcBufs {
   int fp16;     // slices are fp16 (else bf16)
 };
 
+// Blocks per unit of the packing launches: the operators of a superblock are
+// tens of thousands of units, four blocks each fill the GPU; psi is a few
+// dozen sectors of up to a million elements, which four blocks each left to
+// 2 % of the threads (18 orbitals, M=1000: 289 us for 40 MB).
+inline int pack_split(int nunits) { return nunits >= 1024 ? 4 : nunits > 64 ? 4096 / nunits : 64; }
 cudaError_t launch_tc_pack(const TcBufs& b, const TcPack* units, int nunits, cudaStream_t s);
 // phase 1 or 2 on nblocks persistent blocks: block j runs the work records
 // work[ranges[j].x .. ranges[j].y); nb = output-tile width (kTcRowsB or

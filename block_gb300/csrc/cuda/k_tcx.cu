@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(256) tcx_rowexp_kernel(TcxBufs b, const TcPack
   int* ex = pick_x(b.ex, u.pool) + u.ex_off;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (!u.trans) {
-    for (int r = warp; r < u.rows_p; r += 8) {
+    for (int r = warp + 8 * blockIdx.y; r < u.rows_p; r += 8 * gridDim.y) {
       int m = kTcxNoExp;
       if (r < u.rows_v)
         for (int k = lane; k < u.cols_v; k += 32) m = max(m, exp_of(src[(int64_t)r * u.ld + k]));
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(256) tcx_rowexp_kernel(TcxBufs b, const TcPack
       if (lane == 0) ex[r] = m;
     }
   } else {
-    for (int r = tid; r < u.rows_p; r += 256) {
+    for (int r = tid + 256 * blockIdx.y; r < u.rows_p; r += 256 * gridDim.y) {
       int m = kTcxNoExp;
       if (r < u.rows_v)
         for (int k = 0; k < u.cols_v; ++k) m = max(m, exp_of(src[(int64_t)k * u.ld + r]));
@@ -472,7 +472,16 @@ __global__ void __launch_bounds__(256) tcx_reduce_kernel(const double* __restric
   for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < n; e += gridDim.y * blockDim.x) {
     double acc = 0.0;
     const int r = e / t.w, c = e % t.w;
-    for (int p = t.pbeg; p < t.pend; ++p) acc += partials[slots[p] + (int64_t)r * t.pad + c];
+    const double* src = partials + (int64_t)r * t.pad + c;
+    int p = t.pbeg;
+    for (; p + 8 <= t.pend; p += 8) {  // eight partials in flight, summed in slot order
+      double v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = src[slots[p + i]];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc += v[i];
+    }
+    for (; p < t.pend; ++p) acc += src[slots[p]];
     sigma[t.s_off + (int64_t)(t.r0 + r) * t.lds + t.c0 + c] = acc;
   }
 }
@@ -482,12 +491,12 @@ __global__ void fill_int_kernel(int* x, int64_t n, int v) {
 }
 
 cudaError_t launch_tcx_rowexp(const TcxBufs& b, const TcPack* units, int nunits, cudaStream_t s) {
-  if (nunits > 0) tcx_rowexp_kernel<<<nunits, 256, 0, s>>>(b, units);
+  if (nunits > 0) tcx_rowexp_kernel<<<dim3(nunits, nunits >= 1024 ? 1 : 8), 256, 0, s>>>(b, units);
   return cudaGetLastError();
 }
 
 cudaError_t launch_tcx_pack(const TcxBufs& b, const TcPack* units, int nunits, cudaStream_t s) {
-  if (nunits > 0) tcx_pack_kernel<<<dim3(nunits, 4), 256, 0, s>>>(b, units);
+  if (nunits > 0) tcx_pack_kernel<<<dim3(nunits, pack_split(nunits)), 256, 0, s>>>(b, units);
   return cudaGetLastError();
 }
 
@@ -512,7 +521,7 @@ int tcx_blocks_per_sm() { return 1; }
 
 cudaError_t launch_tcx_reduce(const TcxBufs& b, const TcTile* tiles, const int64_t* slots, int ntiles, double* sigma,
                               cudaStream_t s) {
-  if (ntiles > 0) tcx_reduce_kernel<<<dim3(ntiles, 16), 256, 0, s>>>(b.partials, tiles, slots, sigma);
+  if (ntiles > 0) tcx_reduce_kernel<<<dim3(ntiles, 32), 256, 0, s>>>(b.partials, tiles, slots, sigma);
   return cudaGetLastError();
 }
 
