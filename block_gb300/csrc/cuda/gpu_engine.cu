@@ -3925,8 +3925,6 @@ int* GpuEngine::eigh_batched(const std::vector<int>& dims, double* a, const std:
     work += (int64_t)n * n;
     J.s_off = work;
     work += dev::eig_scalar_elems(n);
-    J.tile0 = tiles;
-    tiles += J.nt * (J.nt + 1) / 2;
     J.bt0 = bt;
     bt += (n + bt_cols - 1) / bt_cols;
   }
@@ -3942,7 +3940,26 @@ int* GpuEngine::eigh_batched(const std::vector<int>& dims, double* a, const std:
   DevArray<dev::EigJob> dj;
   dj.upload(jobs, stream_);
   dev::EigBufs eb{copy_inputs ? wk : a, z, w, wk, status};
-  cuda_check(dev::launch_eig_tridiag(eb, dj.d, nj, max_n, tiles, stream_), "eigensolver tridiagonalisation");
+  // Tridiagonalisation: orders that fit a cluster's shared memory in one
+  // launch, largest first; the larger ones with two launches a column.
+  std::vector<dev::EigJob> small, big;
+  for (const dev::EigJob& J : jobs) (J.n <= dev::eig_cluster_max_n() ? small : big).push_back(J);
+  std::stable_sort(small.begin(), small.end(), [](const dev::EigJob& x, const dev::EigJob& y) { return x.n > y.n; });
+  std::vector<int> small_n;
+  for (const dev::EigJob& J : small) small_n.push_back(J.n);
+  for (dev::EigJob& J : big) {
+    J.tile0 = tiles;
+    tiles += J.nt * (J.nt + 1) / 2;
+  }
+  DevArray<dev::EigJob> dsmall, dbig;
+  dsmall.upload(small, stream_);
+  dbig.upload(big, stream_);
+  cuda_check(dev::launch_eig_tridiag_cluster(eb, dsmall.d, small_n.data(), (int)small.size(), stream_),
+             "eigensolver tridiagonalisation (clusters)");
+  cuda_check(dev::launch_eig_tridiag(eb, dbig.d, (int)big.size(), max_n, tiles, stream_),
+             "eigensolver tridiagonalisation");
+  dsmall.release(stream_);
+  dbig.release(stream_);
   tridiagonal_dc(jobs, dj.d, wk, status);
   cuda_check(dev::launch_eig_backtransform(eb, dj.d, nj, max_n, bt, stream_), "eigensolver back-transformation");
   dj.release(stream_);

@@ -13,7 +13,9 @@
 // its leaves use the implicit QL iteration with the Wilkinson shift of the
 // leading 2 x 2 block (Bowdler, Martin, Reinsch and Wilkinson, "The QR and
 // QL algorithms for symmetric matrices", Numer. Math. 11 (1968) 293-306).
+#include <algorithm>
 #include <cmath>
+#include <vector>
 
 #include "k_eig.cuh"
 
@@ -267,6 +269,192 @@ __global__ void __launch_bounds__(kBtThreads) eig_backtransform(EigBufs b, const
   if (lane == 0) b.w[J.w_off + rank] = lam;
 }
 
+// ---------------------------------------------------------------- clusters
+//
+// The same reduction with the matrix held in the shared memory of one
+// thread-block cluster per job (full symmetric storage, row i in block
+// i mod C), all columns in one launch.  Per column k:
+//   col   every block corrects column k in its rows (the lazy rank-2 update
+//         of step k-1) and stores it into all blocks' shared memory;
+//   upd   while that exchange is under way, the rank-2 update of the block's
+//         trailing rows (it does not need the new reflector);
+//   house every block forms the whole reflector from the exchanged column;
+//   mul   p = A v for the block's rows, stored into all blocks;
+//   w     every block forms w from p.
+// Two cluster barriers a column replace two launches of the whole grid.
+// Bound by the FP64 pipe (3 n^3 / 3 FMAs at 1.7 a clock and SM over C SMs)
+// and, per column, by about 40 dependent FP64 operations of 63 clocks each:
+// sums therefore use four warps (one per quarter of the SM), four rows are
+// reduced across a warp's lanes together, and the scalars are formed by one
+// warp.  Measured: see launch_eig_tridiag.
+constexpr int kClThreads = 512, kClWarps = kClThreads / 32;
+constexpr int kClRows = 4;  // rows per warp at most: C blocks hold 64 C rows
+constexpr int kClSumWarps = 4;
+
+__device__ __forceinline__ void cl_arrive() { __syncwarp(); asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t cl_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cl_size() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+// x into block `rank`'s copy of the shared-memory variable at p
+__device__ __forceinline__ void cl_store(double* p, uint32_t rank, double x) {
+  uint32_t a = (uint32_t)__cvta_generic_to_shared(p), m;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(m) : "r"(a), "r"(rank));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(m), "d"(x) : "memory");
+}
+
+// row stride of the shared matrix: odd, so that a column's rows fall into
+// different banks
+__host__ __device__ inline int cl_ld(int n) { return n | 1; }
+
+__global__ void __launch_bounds__(kClThreads, 1) eig_tridiag_cluster(EigBufs b, const EigJob* __restrict__ jobs) {
+  extern __shared__ double sm[];
+  __shared__ double red[kClSumWarps], sc[4];  // sc: scale, lead, tau, K
+  const uint32_t C = cl_size(), rank = cl_rank();
+  const EigJob J = jobs[blockIdx.x / C];
+  const int n = J.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const Scal S = scal(b, J);
+  const double* __restrict__ A = b.a + J.a_off;
+  double* __restrict__ V = b.work + J.v_off;
+  if (n == 1) {  // the whole cluster
+    if (rank == 0 && tid == 0) {
+      S.d[0] = A[0];
+      S.e[0] = 0.0;
+    }
+    return;
+  }
+  const int ld = cl_ld(n), rows = (n - (int)rank + (int)C - 1) / (int)C;  // rows rank, rank + C, ..
+  double *v = sm, *w = sm + n, *col = sm + 2 * n, *p = sm + 3 * n, *a = sm + 4 * n;
+  for (int r = warp; r < rows; r += kClWarps) {
+    const int i = r * (int)C + (int)rank;
+    for (int j = lane; j < n; j += 32) a[r * ld + j] = j <= i ? A[(int64_t)i * n + j] : A[(int64_t)j * n + i];
+  }
+  for (int i = tid; i < n; i += kClThreads) v[i] = w[i] = 0.0;  // step 0 has no update behind it
+  cl_arrive();
+  cl_wait();  // every block runs before its shared memory is written
+  // first local row of global row i or above
+  auto first = [&](int i) { return max(0, (i - (int)rank + (int)C - 1) / (int)C); };
+  for (int k = 0; k <= n - 2; ++k) {
+    // column k of A^(k), rows k..n-1
+    const int rk = first(k);
+    if (tid < rows - rk) {
+      const int r = rk + tid, i = r * (int)C + (int)rank;
+      double c = a[r * ld + k];
+      c -= v[i] * w[k] + w[i] * v[k];
+      for (uint32_t q = 0; q < C; ++q) cl_store(col + i, q, c);
+    }
+    cl_arrive();
+    // rank-2 update of the trailing rows and columns k+1..
+    const int r1 = first(k + 1);
+    if (k > 0) {
+      for (int r = r1 + warp; r < rows; r += kClWarps) {
+        const int i = r * (int)C + (int)rank;
+        const double vi = v[i], wi = w[i];
+        double* row = a + r * ld;
+        for (int j = k + 1 + lane; j < n; j += 32) row[j] = fma(-wi, v[j], fma(-vi, w[j], row[j]));
+      }
+    }
+    cl_wait();
+    if (k == n - 2) break;
+    // reflector
+    if (warp < kClSumWarps) {
+      double ss = 0.0;
+      for (int i = k + 2 + tid; i < n; i += 32 * kClSumWarps) ss = fma(col[i], col[i], ss);
+      ss = warp_sum(ss);
+      if (lane == 0) red[warp] = ss;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const double ss = (red[0] + red[1]) + (red[2] + red[3]);
+      const double alpha = col[k + 1];
+      const double xn = sqrt(fma(alpha, alpha, ss));
+      const double beta = -copysign(xn, alpha);
+      // lane 0: tau = (beta - alpha) / beta, lane 1: scale = 1 / (alpha - beta)
+      const double num = lane == 0 ? beta - alpha : 1.0, den = lane == 0 ? beta : alpha - beta;
+      const double q = xn != 0.0 ? num / den : 0.0;
+      if (lane == 0) {
+        sc[2] = q;
+        sc[1] = xn != 0.0 ? 1.0 : 0.0;
+        if (rank == 0) {
+          S.d[k] = col[k];
+          S.e[k] = xn != 0.0 ? beta : 0.0;
+          S.tau[k] = q;
+        }
+      } else if (lane == 1) {
+        sc[0] = q;
+      }
+    }
+    __syncthreads();
+    for (int i = k + 1 + tid; i < n; i += kClThreads) {
+      const double x = i == k + 1 ? sc[1] : col[i] * sc[0];
+      v[i] = x;
+      if ((uint32_t)i % C == rank) V[(int64_t)k * n + i] = x;
+    }
+    __syncthreads();
+    // p = A v, the block's rows
+    {
+      double acc[kClRows] = {};
+#pragma unroll
+      for (int q = 0; q < kClRows; ++q) {
+        const int r = r1 + warp + kClWarps * q;
+        if (r < rows) {
+          const double* row = a + r * ld;
+          for (int j = k + 1 + lane; j < n; j += 32) acc[q] = fma(row[j], v[j], acc[q]);
+        }
+      }
+      // four sums across the lanes at once: lanes with bit 4 take rows 2, 3,
+      // lanes with bit 3 the odd one of their two
+      if (r1 + warp < rows) {  // warp-uniform
+        const bool hi = lane & 16, odd = lane & 8;
+        double x0 = hi ? acc[2] : acc[0], x1 = hi ? acc[3] : acc[1];
+        x0 += __shfl_xor_sync(0xffffffffu, hi ? acc[0] : acc[2], 16);
+        x1 += __shfl_xor_sync(0xffffffffu, hi ? acc[1] : acc[3], 16);
+        double x = odd ? x1 : x0;
+        x += __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 8);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        const int r = r1 + warp + kClWarps * ((hi ? 2 : 0) + (odd ? 1 : 0));
+        if (r < rows)
+          for (uint32_t q = lane & 7; q < C; q += 8) cl_store(p + r * (int)C + (int)rank, q, x);
+      }
+    }
+    cl_arrive();
+    cl_wait();
+    // w = tau p - (tau / 2) (tau p . v) v
+    const double t = sc[2];
+    if (warp < kClSumWarps) {
+      double pv = 0.0;
+      for (int i = k + 1 + tid; i < n; i += 32 * kClSumWarps) pv = fma(p[i], v[i], pv);
+      pv = warp_sum(pv);
+      if (lane == 0) red[warp] = pv;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const double pv = (red[0] + red[1]) + (red[2] + red[3]);
+      if (lane == 0) sc[3] = 0.5 * t * (t * pv);
+    }
+    __syncthreads();
+    const double K = sc[3];
+    for (int i = k + 1 + tid; i < n; i += kClThreads) w[i] = fma(-K, v[i], t * p[i]);
+    __syncthreads();
+  }
+  // last 2 x 2 block (the update of step n-3 has been applied to its rows)
+  if (tid == 0 && (uint32_t)(n - 1) % C == rank) {
+    S.d[n - 2] = col[n - 2];
+    S.e[n - 2] = col[n - 1];
+    S.d[n - 1] = a[(rows - 1) * ld + n - 1];
+    S.e[n - 1] = 0.0;
+    S.tau[n - 2] = 0.0;
+  }
+}
+
 }  // namespace
 
 // One CTA per matrix, one warp per eigenvector: the vector's largest
@@ -322,6 +510,63 @@ cudaError_t launch_eig_tridiag(const EigBufs& b, const EigJob* jobs, int njobs, 
     if (k <= max_n - 3 && tiles > 0) eig_update<<<tiles, kUpdThreads, 0, s>>>(b, jobs, njobs, k);
     if (max_n < 2) break;
   }
+  return cudaGetLastError();
+}
+
+namespace {
+size_t cl_smem(int n, int c) { return ((size_t)4 * n + (size_t)((n + c - 1) / c) * cl_ld(n)) * sizeof(double); }
+constexpr size_t kClSmemMax = 226 * 1024;
+}  // namespace
+
+int eig_cluster_max_n() {
+  int n = 1;
+  while (cl_smem(n + 1, 16) <= kClSmemMax && (n + 1 + 15) / 16 <= kClRows * kClWarps) ++n;
+  return n;
+}
+
+// Cluster size for a batch (orders in descending order): 8 blocks (15 such
+// clusters fit the GPU) or 16 (7 clusters, for orders whose matrix needs
+// them or whose FP64 work decides), by the time of the jobs dealt to the free
+// clusters in order; a job takes n^3 / 1.7 C clocks of FMAs and about 5000 a
+// column for the exchanges and scalars.
+static int eig_cluster_size(const int* dims, int njobs) {
+  auto makespan = [&](int c, int slots) {
+    std::vector<double> t(std::min(slots, njobs), 0.0);
+    for (int j = 0; j < njobs; ++j) {
+      const double n = dims[j];
+      *std::min_element(t.begin(), t.end()) += n * n * n / (1.7 * c) + 5000.0 * n;
+    }
+    return *std::max_element(t.begin(), t.end());
+  };
+  const int n = dims[0];
+  if (cl_smem(n, 8) > kClSmemMax || (n + 7) / 8 > kClRows * kClWarps) return 16;
+  return makespan(16, 7) < makespan(8, 15) ? 16 : 8;
+}
+
+cudaError_t launch_eig_tridiag_cluster(const EigBufs& b, const EigJob* jobs, const int* dims, int njobs,
+                                       cudaStream_t s) {
+  if (njobs <= 0) return cudaSuccess;
+  if (dims[0] < 1 || dims[0] > eig_cluster_max_n()) return cudaErrorInvalidValue;
+  const int c = eig_cluster_size(dims, njobs);
+  const size_t smem = cl_smem(dims[0], c);
+  cudaError_t e = cudaFuncSetAttribute(eig_tridiag_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(eig_tridiag_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(c * njobs));
+  cfg.blockDim = dim3(kClThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)c;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, eig_tridiag_cluster, b, jobs);
+  if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
 

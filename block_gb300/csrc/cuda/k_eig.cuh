@@ -67,6 +67,12 @@ struct EigBufs {
 };
 cudaError_t launch_eig_tridiag(const EigBufs& b, const EigJob* jobs, int njobs, int max_n, int tiles,
                                cudaStream_t s);
+// The same for matrices of order at most eig_cluster_max_n(), each held in the
+// shared memory of a thread-block cluster, in one launch; dims (host): the
+// jobs' orders, in descending order.
+int eig_cluster_max_n();
+cudaError_t launch_eig_tridiag_cluster(const EigBufs& b, const EigJob* jobs, const int* dims, int njobs,
+                                       cudaStream_t s);
 // Eigenvector signs made canonical: in matrix q (order dims[q] at V +
 // off[q], eigenvectors as columns, column-major when colmajor[q] else
 // row-major) every eigenvector's largest component (the first of equal

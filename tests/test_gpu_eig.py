@@ -84,3 +84,26 @@ def test_order_limit_is_refused(gpu_ctx):
 
     with pytest.raises(block_gb300.BgpuError, match="order"):
         gpu_ctx.diagonalise([np.eye(4097)], vectors=False)
+
+
+@pytest.mark.parametrize("n", [4, 7, 8, 9, 15, 16, 17, 33, 463, 464, 465, 640, 641, 642])
+def test_orders_around_the_cluster_sizes(gpu_ctx, n):
+    """Orders at the edges of the cluster reduction: fewer rows than blocks,
+    the largest held by 8 and by 16 blocks, the first that is not held."""
+    rng = np.random.default_rng(n)
+    X = rng.standard_normal((n, n))
+    A = 0.5 * (X + X.T)
+    (w, V), = gpu_ctx.diagonalise([A])
+    check(A, w, V)
+
+
+def test_batch_larger_than_the_resident_clusters(gpu_ctx):
+    """More matrices than clusters fit the GPU at once, small and held ones
+    and one beyond the limit, in an order that is not sorted."""
+    rng = np.random.default_rng(3)
+    mats = []
+    for n in [20, 300, 1, 2, 3] * 5 + [700] + [61] * 20:
+        X = rng.standard_normal((n, n))
+        mats.append(0.5 * (X + X.T))
+    for A, (w, V) in zip(mats, gpu_ctx.diagonalise(mats)):
+        check(A, w, V)
