@@ -810,9 +810,11 @@ int bgpu_diagonalise(bgpu_ctx* ctx, int nmat, const int* dims, const double* a, 
     cuda_check(cudaMemcpyAsync(da, a, ta * sizeof(double), cudaMemcpyHostToDevice, e.stream()), "h2d");
     int* st = e.eigh_batched(d, da, aoff, /*copy_inputs=*/false, dz, aoff, dw, woff);
     std::vector<int> hs(nmat);
-    std::vector<double> z(eigvecs ? ta : 0);
     cuda_check(cudaMemcpyAsync(eigvals, dw, tw * sizeof(double), cudaMemcpyDeviceToHost, e.stream()), "d2h");
-    if (eigvecs) cuda_check(cudaMemcpyAsync(z.data(), dz, ta * sizeof(double), cudaMemcpyDeviceToHost, e.stream()), "d2h");
+    if (eigvecs) {  // column-major per matrix -> row-major with the eigenvectors as columns, into the spent inputs
+      e.transpose_batched(dz, da, aoff, d);
+      cuda_check(cudaMemcpyAsync(eigvecs, da, ta * sizeof(double), cudaMemcpyDeviceToHost, e.stream()), "d2h");
+    }
     cuda_check(cudaMemcpyAsync(hs.data(), st, nmat * sizeof(int), cudaMemcpyDeviceToHost, e.stream()), "d2h");
     e.sync();
     cudaFreeAsync(st, e.stream());
@@ -822,14 +824,6 @@ int bgpu_diagonalise(bgpu_ctx* ctx, int nmat, const int* dims, const double* a, 
     for (int j = 0; j < nmat; ++j)
       if (hs[j] < 0) throw std::runtime_error("bgpu_diagonalise: tridiagonal solver did not converge for matrix " +
                                               std::to_string(j));
-    if (eigvecs)  // column-major per matrix -> row-major with the eigenvectors as columns
-      for (int j = 0; j < nmat; ++j) {
-        const int n = d[j];
-        const double* src = z.data() + aoff[j];
-        double* dst = eigvecs + aoff[j];
-        for (int r = 0; r < n; ++r)
-          for (int c = 0; c < n; ++c) dst[(int64_t)r * n + c] = src[(int64_t)c * n + r];
-      }
   });
 }
 

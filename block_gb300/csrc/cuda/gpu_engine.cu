@@ -147,6 +147,9 @@ GpuEngine::GpuEngine(int device) : device_(device) {
   cuda_check(cudaDeviceGetDefaultMemPool(&pool, device_), "mempool");
   uint64_t thr = UINT64_MAX;
   cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
+  cuda_check(cudaStreamCreateWithFlags(&side_stream_, cudaStreamNonBlocking), "stream");
+  cuda_check(cudaEventCreateWithFlags(&side_fork_, cudaEventDisableTiming), "event");
+  cuda_check(cudaEventCreateWithFlags(&side_join_, cudaEventDisableTiming), "event");
   cuda_check(cudaEventCreate(&ev0_), "event");
   cuda_check(cudaEventCreate(&ev1_), "event");
   cuda_check(cudaMalloc((void**)&tc_status_, sizeof(int)), "alloc status");
@@ -179,6 +182,9 @@ GpuEngine::~GpuEngine() {
     if (q) cudaFreeAsync(q, stream_);
   cudaStreamSynchronize(stream_);
   release_staging(stream_);
+  cudaStreamDestroy(side_stream_);
+  cudaEventDestroy(side_fork_);
+  cudaEventDestroy(side_join_);
   cudaEventDestroy(ev0_);
   cudaEventDestroy(ev1_);
   cudaFree(tc_status_);
@@ -497,6 +503,20 @@ void add_tasks(std::vector<dev::GemmTask>& t, int unit, int m, int n, int tile =
 }  // namespace
 
 // ------------------------------------------------------------------ build
+
+// Tasks of whole units; returns the tile edge.  Lists that do not give every
+// SM a tile of 32 x 32 are cut into 16 x 16 tiles: a tile is a serial chain
+// over its K (0.3 us per row of K at 32 x 32; 54 tiles of an order-259 merge:
+// 81 -> 57 us).  Longer lists are faster with the larger tile, which loads
+// half as much per product (460 tiles up to order 400: 347 against 474 us).
+int GpuEngine::list_tasks(std::vector<dev::GemmTask>& t, const std::vector<dev::GemmUnit>& units) {
+  int64_t n = 0;
+  for (const auto& u : units)
+    n += (int64_t)((u.m + dev::kGemmTile - 1) / dev::kGemmTile) * ((u.n + dev::kGemmTile - 1) / dev::kGemmTile);
+  const int edge = n < sm_count() ? dev::kGemmTileSmall : dev::kGemmTile;
+  for (int u = 0; u < (int)units.size(); ++u) add_tasks(t, u, units[u].m, units[u].n, edge);
+  return edge;
+}
 
 void GpuEngine::build_block(Block& big, const Block& a, const Block& b,
                             const std::vector<std::pair<OpKey, std::vector<BuildTerm>>>& recipes) {
@@ -1556,6 +1576,9 @@ void GpuEngine::plan_tc(const Superblock& sb, SigmaPlan& plan) {
     plan.tc_pool_cap[i] = cap;
   }
   plan.tc_psi_pack.upload(psi_packs, stream_);
+  int64_t psi_most = 0;
+  for (const TcPack& p : psi_packs) psi_most = std::max(psi_most, (int64_t)p.rows_p * p.kp);
+  plan.tc_psi_split = unit_split(psi_most, 8);
   plan.tc_rows.upload(rows_tab, stream_);
   // operator blocks are packed once per plan
   DevArray<TcPack> dops;
@@ -2066,6 +2089,9 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
   plan.tc_r1.upload(wr1, stream_);
   plan.tc_r2.upload(wr2, stream_);
   plan.tc_tiles.upload(tiles, stream_);
+  int64_t tile_most = 0;
+  for (const TcTile& t : tiles) tile_most = std::max(tile_most, (int64_t)t.h * t.w);
+  plan.tc_tile_split = unit_split(tile_most, 1);
   plan.tc_slots.upload(slots, stream_);
   plan.tc_mma_flops = mma;
   plan.tc_l1 = std::move(l1);
@@ -2247,7 +2273,7 @@ void GpuEngine::sigma_tc(const Superblock& sb, SigmaPlan& p, const double* psi, 
   b.status = tc_status_;
   b.fp16 = fp16 ? 1 : 0;
   constexpr uint64_t kWaitLimitNs = 1000000000ull;
-  cuda_check(dev::launch_tc_pack(b, p.tc_psi_pack.d, (int)p.tc_psi_pack.n, stream_), "tc pack psi");
+  cuda_check(dev::launch_tc_pack(b, p.tc_psi_pack.d, (int)p.tc_psi_pack.n, stream_, p.tc_psi_split), "tc pack psi");
   if (marks) cuda_check(cudaEventRecord(marks[0], stream_), "record");
   if (p.tc_knobs.per_sector) {
     // baseline: one launch per psi sector (phase 1) and per sigma sector
@@ -2269,7 +2295,7 @@ void GpuEngine::sigma_tc(const Superblock& sb, SigmaPlan& p, const double* psi, 
                  "tc phase 2");
   }
   if (marks) cuda_check(cudaEventRecord(marks[1], stream_), "record");
-  cuda_check(dev::launch_tc_reduce(b, p.tc_tiles.d, p.tc_slots.d, (int)p.tc_tiles.n, out, stream_), "tc reduce");
+  cuda_check(dev::launch_tc_reduce(b, p.tc_tiles.d, p.tc_slots.d, (int)p.tc_tiles.n, out, stream_, p.tc_tile_split), "tc reduce");
   if (p.ecore != 0.0) cuda_check(dev::launch_axpy(p.ecore, psi, out, p.n, stream_), "ecore");
   cuda_check(cudaMemcpyAsync(tc_status_host_, tc_status_, sizeof(int), cudaMemcpyDeviceToHost, stream_), "status");
   sigma_flops += p.flops;
@@ -2295,8 +2321,8 @@ void GpuEngine::sigma_tcx(const Superblock& sb, SigmaPlan& p, const double* psi,
   b.partials = reinterpret_cast<double*>(p.tc_partials);
   b.status = tc_status_;
   constexpr uint64_t kWaitLimitNs = 1000000000ull;
-  cuda_check(dev::launch_tcx_rowexp(b, p.tc_psi_pack.d, (int)p.tc_psi_pack.n, stream_), "tcx psi exponents");
-  cuda_check(dev::launch_tcx_pack(b, p.tc_psi_pack.d, (int)p.tc_psi_pack.n, stream_), "tcx pack psi");
+  cuda_check(dev::launch_tcx_rowexp(b, p.tc_psi_pack.d, (int)p.tc_psi_pack.n, stream_, p.tc_psi_split), "tcx psi exponents");
+  cuda_check(dev::launch_tcx_pack(b, p.tc_psi_pack.d, (int)p.tc_psi_pack.n, stream_, p.tc_psi_split), "tcx pack psi");
   cuda_check(dev::launch_fill_int(p.tcx_ex[dev::kTcPoolS], p.tcx_ex_n[dev::kTcPoolS], dev::kTcxNoExp, stream_),
              "tcx T exponents");
   cuda_check(dev::launch_tcx_sigma(1, b, p.tcx_w1.d, p.tc_r1.d, (int)p.tc_r1.n, out, kWaitLimitNs, stream_),
@@ -2304,7 +2330,7 @@ void GpuEngine::sigma_tcx(const Superblock& sb, SigmaPlan& p, const double* psi,
   cuda_check(dev::launch_tcx_pack(b, p.tcx_tpack.d, (int)p.tcx_tpack.n, stream_), "tcx pack T");
   cuda_check(dev::launch_tcx_sigma(2, b, p.tcx_w2.d, p.tc_r2.d, (int)p.tc_r2.n, out, kWaitLimitNs, stream_),
              "tcx phase 2");
-  cuda_check(dev::launch_tcx_reduce(b, p.tc_tiles.d, p.tc_slots.d, (int)p.tc_tiles.n, out, stream_), "tcx reduce");
+  cuda_check(dev::launch_tcx_reduce(b, p.tc_tiles.d, p.tc_slots.d, (int)p.tc_tiles.n, out, stream_, p.tc_tile_split), "tcx reduce");
   if (p.ecore != 0.0) cuda_check(dev::launch_axpy(p.ecore, psi, out, p.n, stream_), "ecore");
   cuda_check(cudaMemcpyAsync(tc_status_host_, tc_status_, sizeof(int), cudaMemcpyDeviceToHost, stream_), "status");
   sigma_flops += p.flops;
@@ -3463,6 +3489,16 @@ std::string GpuEngine::step_stats() {
 
 // ------------------------------------------------------------------ density
 
+namespace {
+// waits for the second stream when an error leaves before it was joined
+struct SideJoin {
+  cudaStream_t s;
+  ~SideJoin() {
+    if (s) cudaStreamSynchronize(s);
+  }
+};
+}  // namespace
+
 void GpuEngine::density(const Superblock& sb, bool left, const std::vector<double>& weights, DensitySpectrum& spec) {
   PlanLaps laps{"density"};
   const Block& B = left ? *sb.L : *sb.R;
@@ -3518,7 +3554,7 @@ void GpuEngine::density(const Superblock& sb, bool left, const std::vector<doubl
     u.iend = (int)items.size();
     units.push_back(u);
   }
-  for (int u = 0; u < (int)units.size(); ++u) add_tasks(tasks, u, units[u].m, units[u].n);
+  const int edge = list_tasks(tasks, units);
   DevArray<dev::GemmUnit> du;
   DevArray<dev::GemmItem> di;
   DevArray<dev::GemmTask> dt;
@@ -3528,7 +3564,7 @@ void GpuEngine::density(const Superblock& sb, bool left, const std::vector<doubl
   dev::Bufs bufs{};
   bufs.p[0] = waves_;
   bufs.p[1] = rho;
-  cuda_check(dev::launch_gemm(bufs, du.d, di.d, dt.d, (int)tasks.size(), stream_), "density");
+  cuda_check(dev::launch_gemm(bufs, du.d, di.d, dt.d, (int)tasks.size(), stream_, edge), "density");
   if (noise_.any()) add_noise(sb, left, rho, off);
   if (laps.on) sync();
   laps.lap("rho gemm");
@@ -3563,11 +3599,19 @@ void GpuEngine::density(const Superblock& sb, bool left, const std::vector<doubl
   ddims.upload(small_dims, stream_);
   dstat.upload(std::vector<int>(nq, 0), stream_);
   double* jac = nullptr;  // the Jacobi sweeps overwrite their matrices: a copy of rho
+  // The small sectors' Jacobi sweeps (one block each) run on a second stream
+  // beside the large sectors' solver; both write their own sectors.  Every
+  // buffer belongs to stream_, which waits for the sweeps before it goes on.
+  SideJoin side{side_stream_};
   if (small_max > 0) {
     jac = alloc(tot);
     cuda_check(cudaMemcpyAsync(jac, rho, tot * sizeof(double), cudaMemcpyDeviceToDevice, stream_), "copy rho");
-    cuda_check(dev::launch_jacobi(jac, doff.d, ddims.d, w, dwoff.d, dm_vecs_, doff.d, dstat.d, nq, small_max, stream_),
+    cuda_check(cudaEventRecord(side_fork_, stream_), "record");
+    cuda_check(cudaStreamWaitEvent(side_stream_, side_fork_, 0), "wait");
+    cuda_check(dev::launch_jacobi(jac, doff.d, ddims.d, w, dwoff.d, dm_vecs_, doff.d, dstat.d, nq, small_max,
+                                  side_stream_),
                "density eig");
+    cuda_check(cudaEventRecord(side_join_, side_stream_), "record");
   }
   int* eig_status = nullptr;
   if (!large.empty()) {
@@ -3583,6 +3627,8 @@ void GpuEngine::density(const Superblock& sb, bool left, const std::vector<doubl
     }
     eig_status = eigh_batched(dims, rho, aoff, /*copy_inputs=*/true, dm_vecs_, zoff, w, wo);
   }
+  if (small_max > 0) cuda_check(cudaStreamWaitEvent(stream_, side_join_, 0), "wait");
+  side.s = nullptr;  // joined
   {
     // eigenvector signs as on every engine (the basis of the renormalised
     // block, and so the random noise of later steps, depends on them)
@@ -3909,7 +3955,6 @@ int* GpuEngine::eigh_batched(const std::vector<int>& dims, double* a, const std:
   if (max_n > dev::kEigMaxN)
     throw std::runtime_error("eigensolver: matrix of order " + std::to_string(max_n) + " above the limit " +
                              std::to_string(dev::kEigMaxN));
-  const int bt_cols = dev::eig_bt_cols(max_n);
   for (int j = 0; j < nj; ++j) {
     dev::EigJob& J = jobs[j];
     const int n = dims[j];
@@ -3925,8 +3970,6 @@ int* GpuEngine::eigh_batched(const std::vector<int>& dims, double* a, const std:
     work += (int64_t)n * n;
     J.s_off = work;
     work += dev::eig_scalar_elems(n);
-    J.bt0 = bt;
-    bt += (n + bt_cols - 1) / bt_cols;
   }
   double* wk = alloc(work);
   if (copy_inputs)
@@ -3940,31 +3983,47 @@ int* GpuEngine::eigh_batched(const std::vector<int>& dims, double* a, const std:
   DevArray<dev::EigJob> dj;
   dj.upload(jobs, stream_);
   dev::EigBufs eb{copy_inputs ? wk : a, z, w, wk, status};
-  // Tridiagonalisation: orders that fit a cluster's shared memory in one
-  // launch, largest first; the larger ones with two launches a column.
-  std::vector<dev::EigJob> small, big;
-  for (const dev::EigJob& J : jobs) (J.n <= dev::eig_cluster_max_n() ? small : big).push_back(J);
-  std::stable_sort(small.begin(), small.end(), [](const dev::EigJob& x, const dev::EigJob& y) { return x.n > y.n; });
+  // The jobs by descending order: the largest start first in the
+  // tridiagonalisation (orders that fit a cluster's shared memory in one
+  // launch, the larger ones with two launches a column) and in the
+  // back-transformation.
+  std::vector<dev::EigJob> sorted = jobs;
+  std::stable_sort(sorted.begin(), sorted.end(), [](const dev::EigJob& x, const dev::EigJob& y) { return x.n > y.n; });
+  int nbig = 0;
   std::vector<int> small_n;
-  for (const dev::EigJob& J : small) small_n.push_back(J.n);
-  for (dev::EigJob& J : big) {
-    J.tile0 = tiles;
-    tiles += J.nt * (J.nt + 1) / 2;
+  for (dev::EigJob& J : sorted) {
+    if (J.n > dev::eig_cluster_max_n()) {
+      J.tile0 = tiles;
+      tiles += J.nt * (J.nt + 1) / 2;
+      ++nbig;
+    } else {
+      small_n.push_back(J.n);
+    }
+    J.bt0 = bt;
+    bt += (J.n + dev::kEigBtCols - 1) / dev::kEigBtCols;
   }
-  DevArray<dev::EigJob> dsmall, dbig;
-  dsmall.upload(small, stream_);
-  dbig.upload(big, stream_);
-  cuda_check(dev::launch_eig_tridiag_cluster(eb, dsmall.d, small_n.data(), (int)small.size(), stream_),
+  DevArray<dev::EigJob> dsorted;
+  dsorted.upload(sorted, stream_);
+  cuda_check(dev::launch_eig_tridiag(eb, dsorted.d, nbig, max_n, tiles, stream_), "eigensolver tridiagonalisation");
+  cuda_check(dev::launch_eig_tridiag_cluster(eb, dsorted.d + nbig, small_n.data(), nj - nbig, stream_),
              "eigensolver tridiagonalisation (clusters)");
-  cuda_check(dev::launch_eig_tridiag(eb, dbig.d, (int)big.size(), max_n, tiles, stream_),
-             "eigensolver tridiagonalisation");
-  dsmall.release(stream_);
-  dbig.release(stream_);
   tridiagonal_dc(jobs, dj.d, wk, status);
-  cuda_check(dev::launch_eig_backtransform(eb, dj.d, nj, max_n, bt, stream_), "eigensolver back-transformation");
+  cuda_check(dev::launch_eig_backtransform(eb, dsorted.d, nj, max_n, bt, stream_), "eigensolver back-transformation");
   dj.release(stream_);
+  dsorted.release(stream_);
   free(wk);
   return status;
+}
+
+void GpuEngine::transpose_batched(const double* a, double* t, const std::vector<int64_t>& off,
+                                  const std::vector<int>& dims) {
+  DevArray<int64_t> doff;
+  DevArray<int> dd;
+  doff.upload(off, stream_);
+  dd.upload(dims, stream_);
+  cuda_check(dev::launch_transpose(a, t, doff.d, dd.d, (int)dims.size(), stream_), "transpose");
+  doff.release(stream_);
+  dd.release(stream_);
 }
 
 // Divide and conquer on the tridiagonal matrices of an eigensolver batch
@@ -4081,7 +4140,7 @@ void GpuEngine::tridiagonal_dc(const std::vector<dev::EigJob>& jobs, const dev::
       u.iend = (int)items.size();
       units.push_back(u);
     }
-    for (int u = 0; u < (int)units.size(); ++u) add_tasks(tasks, u, units[u].m, units[u].n);
+    const int edge = list_tasks(tasks, units);
     if (!tasks.empty()) {
       DevArray<dev::GemmUnit> du;
       DevArray<dev::GemmItem> di;
@@ -4093,7 +4152,7 @@ void GpuEngine::tridiagonal_dc(const std::vector<dev::EigJob>& jobs, const dev::
       bufs.p[0] = L.U;
       bufs.p[1] = L.G;
       bufs.p[2] = wk;
-      cuda_check(dev::launch_gemm(bufs, du.d, di.d, dt.d, (int)tasks.size(), stream_), "merge eigenvectors");
+      cuda_check(dev::launch_gemm(bufs, du.d, di.d, dt.d, (int)tasks.size(), stream_, edge), "merge eigenvectors");
       du.release(stream_);
       di.release(stream_);
       dt.release(stream_);

@@ -116,6 +116,7 @@ struct SigmaPlan {
   __nv_bfloat16* tc_pool[dev::kTcPools] = {};  // packed operands, hi and lo per block
   int64_t tc_pool_elems[dev::kTcPools] = {};
   DevArray<dev::TcPack> tc_psi_pack;
+  int tc_psi_split = 1, tc_tile_split = 1;  // blocks per unit of the psi packing and per tile of the partial sums
   DevArray<dev::TcWork> tc_w1, tc_w2;  // work records of phases 1 and 2, grouped by block
   DevArray<int2> tc_r1, tc_r2;         // per persistent block: its range of records
   DevArray<dev::TcTile> tc_tiles;
@@ -256,6 +257,7 @@ class GpuEngine : public Engine {
   int sigma_launches(const SigmaPlan& plan) const;
   double* arena(const Block& b) const;
   int sm_count();
+  int list_tasks(std::vector<dev::GemmTask>& t, const std::vector<dev::GemmUnit>& units);
   cudaStream_t stream() const { return stream_; }
   double* alloc(int64_t elems);
   void free(double* p);
@@ -276,6 +278,8 @@ class GpuEngine : public Engine {
   // of per-matrix status words for the caller to read and free
   int* eigh_batched(const std::vector<int>& dims, double* a, const std::vector<int64_t>& a_off, bool copy_inputs,
                     double* z, const std::vector<int64_t>& z_off, double* w, const std::vector<int64_t>& w_off);
+  // matrix j of order dims[j] at a + off[j], transposed, to t + off[j]
+  void transpose_batched(const double* a, double* t, const std::vector<int64_t>& off, const std::vector<int>& dims);
   // divide and conquer on the tridiagonal matrices of an eigensolver batch
   void tridiagonal_dc(const std::vector<dev::EigJob>& jobs, const dev::EigJob* djobs, double* wk, int* status);
   int64_t wave_size() const { return wave_n_; }
@@ -358,6 +362,9 @@ class GpuEngine : public Engine {
   std::vector<int64_t> rot_off_;
   std::vector<int> rot_kept_, rot_rows_;
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
+  // second stream (density): forked from and joined to stream_ within a call
+  cudaStream_t side_stream_ = nullptr;
+  cudaEvent_t side_fork_ = nullptr, side_join_ = nullptr;
   // rotation that made each renormalised block (big-block quantum q: n[q] x m[q]
   // row-major at off[q]), kept for the wavefunction guess transform
   struct RotRecord {

@@ -11,7 +11,7 @@ namespace {
 constexpr double kEps = 2.220446049250313e-16;
 constexpr int kLeafWarps = 4;
 constexpr int kDefThreads = 256;
-constexpr int kWarpThreads = 256;  // warps-per-slot kernels: 8 warps per CTA
+constexpr int kWarpThreads = 128;  // warp-per-slot kernels: 4 warps per CTA, one per quarter of an SM
 constexpr int kColThreads = 128;   // CTA-per-column kernels
 constexpr int kSecularIters = 256;
 constexpr int kLeafIters = 60;     // QL sweeps per eigenvalue of a leaf
@@ -30,6 +30,16 @@ __device__ __forceinline__ double warp_max(double x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x = fmax(x, __shfl_xor_sync(0xffffffffu, x, o));
   return x;
+}
+
+// h^-1/2 for normal h: the hardware's approximation y (relative error below
+// 2^-20), then y (1 - r)^-1/2 with r = 1 - h y^2 by the binomial series to
+// second order (error 5 r^3 / 16 below 2^-60 before rounding)
+__device__ __forceinline__ double inv_sqrt(double h) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(h));
+  const double r = fma(-h * y, y, 1.0);
+  return fma(y * r, fma(0.375, r, 0.5), y);
 }
 
 // scalar work area of a job (k_eig.cu): d, e, tau, unsorted eigenvalues, ...
@@ -65,6 +75,12 @@ __global__ void dc_tear_kernel(double* work, const EigJob* __restrict__ jobs, co
 // the large solver, k_eig.cu, in one warp): lane 0 runs the scalar
 // recurrence of one sweep and leaves its rotations in shared memory, then
 // every lane applies them to its row of the leaf's Z.
+// Bound by the recurrence: one thread's FP64 operations issue every 63
+// clocks, so their number counts.  The leaf is scaled by a power of two to
+// norm near one, so that the rotation comes from one reciprocal square root
+// of f^2 + g^2 (about 20 operations a rotation instead of about 60 with
+// hypot and two divisions; leaves of the 12 matrices up to order 400:
+// 1973 -> 1095 us).
 __global__ void __launch_bounds__(32 * kLeafWarps) dc_leaf_kernel(double* work, const EigJob* __restrict__ jobs,
                                                                   const DcLeaf* __restrict__ leaves, int nleaves,
                                                                   int* status) {
@@ -89,12 +105,17 @@ __global__ void __launch_bounds__(32 * kLeafWarps) dc_leaf_kernel(double* work, 
   __syncwarp();
   int l = 0, it = 0;
   bool fail = false;
-  double tiny = 0.0;
-  if (lane == 0) {
-    double tn = 0.0;
-    for (int i = 0; i < len; ++i) tn = fmax(tn, fabs(d[i]) + fabs(e[i]));
-    tiny = kEps * tn;
+  // scaled to norm in [1, 2): squares of anything above 1e-154 of the norm
+  // stay normal, and what is below is negligible against tiny
+  double tn = lane < len ? fabs(d[lane]) + fabs(e[lane]) : 0.0;
+  tn = warp_max(tn);
+  const int ex = tn > 0.0 && tn < 1e308 * 1.7 ? ilogb(tn) : 0;
+  if (lane < len) {
+    d[lane] = scalbn(d[lane], -ex);
+    e[lane] = scalbn(e[lane], -ex);
   }
+  const double tiny = kEps * scalbn(tn, -ex);
+  __syncwarp();
   while (true) {
     if (lane == 0) {
       int m = -1, cnt = 0;
@@ -115,28 +136,30 @@ __global__ void __launch_bounds__(32 * kLeafWarps) dc_leaf_kernel(double* work, 
           m = -1;
           break;
         }
-        double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
-        double r = hypot(g, 1.0);
+        double g = (d[l + 1] - d[l]) / (2.0 * e[l]);  // |e| > tiny: below 1e16
+        double r = sqrt(fma(g, g, 1.0));
         g = d[m] - d[l] + e[l] / (g + copysign(r, g));
         double s = 1.0, c = 1.0, p = 0.0;
         bool early = false;
         for (int i = m - 1; i >= l; --i) {
           const double f = s * e[i], bb = c * e[i];
-          r = hypot(f, g);
-          e[i + 1] = r;
-          if (r == 0.0) {
+          const double h = fma(f, f, g * g);
+          if (__double2hiint(h) < 0x00100000) {  // zero or subnormal: f and g are negligible
+            e[i + 1] = 0.0;
             d[i + 1] -= p;
             e[m] = 0.0;
             early = true;
             break;
           }
-          s = f / r;
-          c = g / r;
+          const double q = inv_sqrt(h);
+          e[i + 1] = h * q;
+          s = f * q;
+          c = g * q;
           g = d[i + 1] - p;
-          r = (d[i] - g) * s + 2.0 * c * bb;
+          r = fma(d[i] - g, s, c * (bb + bb));
           p = s * r;
           d[i + 1] = g + p;
-          g = c * r - bb;
+          g = fma(c, r, -bb);
           rb[w][cnt++] = make_double2(c, s);
         }
         if (!early) {
@@ -168,7 +191,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps) dc_leaf_kernel(double* work, 
     __syncwarp();
   }
   double* __restrict__ Z = work + J.q_off;
-  if (lane < len) eig_of(work, J)[o + lane] = d[lane];
+  if (lane < len) eig_of(work, J)[o + lane] = scalbn(d[lane], ex);
   for (int c = 0; c < len; ++c)
     if (lane < len) Z[(int64_t)(o + c) * n + o + lane] = z[c * kDcLeaf + lane];
   if (lane == 0 && fail) status[Lf.job] = -1;
@@ -190,7 +213,9 @@ __global__ void __launch_bounds__(kDefThreads) dc_deflate_kernel(double* work, c
   while (P < nm) P <<= 1;
   double* key = sm;
   double* zs = sm + P;
-  int* idx = reinterpret_cast<int*>(sm + 2 * P);
+  double* zt = sm + 2 * P;
+  int* idx = reinterpret_cast<int*>(sm + 3 * P);
+  int* kept = idx + P;  // sorted positions of the poles not deflated by their weight
   double* __restrict__ Z = work + J.q_off;
   const double* eu = eig_of(work, J);
   const double beta = offd_of(work, J)[o + n1 - 1];
@@ -238,11 +263,55 @@ __global__ void __launch_bounds__(kDefThreads) dc_deflate_kernel(double* work, c
   __syncthreads();
   double zmax = 0.0;
   for (int i = 0; i < kDefThreads / 32; ++i) zmax = fmax(zmax, red[i]);
+  // Deflation by weight and the test for close neighbours on all threads; the
+  // poles change as they are merged, so only a merge that holds a close pair
+  // takes the serial scan below (about eight FP64 operations of 63 clocks a
+  // pole: 105 of 170 us at order 400, where no pair is close).
+  const int64_t x = M.x_off;
+  const double zsc = zn2 > 0.0 ? 1.0 / sqrt(zn2) : 0.0;
+  const double rho = fabs(beta) * zn2;
+  const double tol = 8.0 * kEps * fmax(fmax(fabs(key[0]), fabs(key[nm - 1])), zmax * zsc);
+  for (int t = tid; t < nm; t += kDefThreads) zt[t] = zs[idx[t]] * zsc;
+  __syncthreads();
+  if (tid < 32) {
+    int cnt = 0;
+    for (int t0 = 0; t0 < nm; t0 += 32) {
+      const int t = t0 + tid;
+      const bool keep = t < nm && !(rho * fabs(zt[t]) <= tol);
+      const unsigned mask = __ballot_sync(0xffffffffu, keep);
+      if (keep) kept[cnt + __popc(mask & ((1u << tid) - 1u))] = t;
+      if (t < nm && !keep) {  // deflated values from the end of the slots, in sorted order
+        const int nd = t0 - cnt + __popc(~mask & ((1u << tid) - 1u));
+        L.dk[x + nm - 1 - nd] = key[t];
+        L.col[x + nm - 1 - nd] = idx[t];
+      }
+      cnt += __popc(mask);
+    }
+    if (tid == 0) nrot_s = cnt;
+  }
+  __syncthreads();
+  const int nkept = nrot_s;
+  bool close = false;
+  for (int m = 1 + tid; m < nkept; m += kDefThreads) {
+    const double pd = key[kept[m - 1]], pz = zt[kept[m - 1]], dt = key[kept[m]], zz = zt[kept[m]];
+    if (fabs((dt - pd) * zz * pz) <= tol * (zz * zz + pz * pz)) close = true;
+  }
+  const bool serial = __syncthreads_or(close) != 0;
+  if (!serial) {
+    for (int m = tid; m < nkept; m += kDefThreads) {
+      const int t = kept[m];
+      L.dk[x + m] = key[t];
+      L.zk[x + m] = zt[t];
+      L.col[x + m] = idx[t];
+    }
+    if (tid == 0) {
+      L.K[blockIdx.x] = nkept;
+      L.nrot[blockIdx.x] = 0;
+      L.rho[blockIdx.x] = rho;
+    }
+    return;
+  }
   if (tid == 0) {
-    const int64_t x = M.x_off;
-    const double zsc = zn2 > 0.0 ? 1.0 / sqrt(zn2) : 0.0;
-    const double rho = fabs(beta) * zn2;
-    const double tol = 8.0 * kEps * fmax(fmax(fabs(key[0]), fabs(key[nm - 1])), zmax * zsc);
     int K = 0, nd = 0, nrot = 0;
     auto pole = [&](double dv, double zv, int cv) {
       L.dk[x + K] = dv;
@@ -261,22 +330,22 @@ __global__ void __launch_bounds__(kDefThreads) dc_deflate_kernel(double* work, c
     for (int t = 0; t < nm; ++t) {
       const double dt = key[t];
       const int ct = idx[t];
-      const double zt = zs[ct] * zsc;
-      if (rho * fabs(zt) <= tol) {
+      const double zv = zt[t];
+      if (rho * fabs(zv) <= tol) {
         deflate(dt, ct);
         continue;
       }
       if (!have) {
         have = true;
         pd = dt;
-        pz = zt;
+        pz = zv;
         pc = ct;
         continue;
       }
       // close pair: |(d_t - d_p) c s| <= tol for the rotation that zeroes z_p
-      const double r2 = zt * zt + pz * pz;
-      if (fabs((dt - pd) * zt * pz) <= tol * r2) {
-        const double tau = sqrt(r2), c = zt / tau, s = -pz / tau;
+      const double r2 = zv * zv + pz * pz;
+      if (fabs((dt - pd) * zv * pz) <= tol * r2) {
+        const double tau = sqrt(r2), c = zv / tau, s = -pz / tau;
         L.rot_cols[x + nrot] = make_int2(pc, ct);
         L.rot_cs[x + nrot] = make_double2(c, s);
         ++nrot;
@@ -287,7 +356,7 @@ __global__ void __launch_bounds__(kDefThreads) dc_deflate_kernel(double* work, c
       } else {
         pole(pd, pz, pc);
         pd = dt;
-        pz = zt;
+        pz = zv;
         pc = ct;
       }
     }
@@ -540,7 +609,7 @@ cudaError_t launch_dc_deflate(double* work, const EigJob* jobs, const DcLevel& L
   if (max_nm < 2 || max_nm > kEigMaxN) return cudaErrorInvalidValue;
   int P = 1;
   while (P < max_nm) P <<= 1;
-  const size_t smem = (size_t)P * (2 * sizeof(double) + sizeof(int));
+  const size_t smem = (size_t)P * (3 * sizeof(double) + 2 * sizeof(int));
   cudaError_t e = cudaFuncSetAttribute(dc_deflate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   dc_deflate_kernel<<<L.nmerges, kDefThreads, smem, s>>>(work, jobs, L);

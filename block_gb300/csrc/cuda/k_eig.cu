@@ -226,9 +226,12 @@ __global__ void __launch_bounds__(kUpdThreads) eig_update(EigBufs b, const EigJo
 
 // Back-transformation V = H_0 H_1 ... H_{n-3} Z, one eigenvector per warp in
 // shared memory, written at the rank of its eigenvalue (ascending; ties in
-// index order).
+// index order).  Four warps a block, one per quarter of the SM, since a
+// warp's FP64 operations issue every 63 clocks; the next reflector is copied
+// while the present one is applied.  12 matrices up to order 400: 1000 ->
+// 846 us (eight warps and two barriers a reflector: fewer, longer blocks).
 __global__ void __launch_bounds__(kBtThreads) eig_backtransform(EigBufs b, const EigJob* __restrict__ jobs,
-                                                                int njobs, int ncol) {
+                                                                int njobs, int max_n) {
   extern __shared__ double sm[];
   const int bid = blockIdx.x;
   const int jidx = find_job(jobs, njobs, bid, 2);
@@ -237,22 +240,30 @@ __global__ void __launch_bounds__(kBtThreads) eig_backtransform(EigBufs b, const
   const Scal S = scal(b, J);
   const double* __restrict__ V = b.work + J.v_off;
   const double* __restrict__ Q = b.work + J.q_off;
-  double* vs = sm;
-  double* zc = sm + n + (int64_t)warp * n;
-  const int j = (bid - J.bt0) * ncol + warp;
-  const bool mine = warp < ncol && j < n;
+  double* zc = sm + (2 + warp) * (int64_t)max_n;
+  const int j = (bid - J.bt0) * kEigBtCols + warp;
+  const bool mine = j < n;
   if (mine)
     for (int i = lane; i < n; i += 32) zc[i] = Q[(int64_t)j * n + i];
+  auto fetch = [&](int k) {  // reflector k into its buffer
+    double* dst = sm + (k & 1) * (int64_t)max_n;
+    for (int i = k + 1 + tid; i < n; i += kBtThreads)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + i)),
+                   "l"(V + (int64_t)k * n + i)
+                   : "memory");
+  };
+  if (n >= 3) fetch(n - 3);
   for (int k = n - 3; k >= 0; --k) {
-    __syncthreads();
-    for (int i = k + 1 + tid; i < n; i += kBtThreads) vs[i] = V[(int64_t)k * n + i];
-    __syncthreads();
-    if (mine) {
-      double dot = 0.0;
-      for (int i = k + 1 + lane; i < n; i += 32) dot += vs[i] * zc[i];
-      dot = warp_sum(dot) * S.tau[k];
-      for (int i = k + 1 + lane; i < n; i += 32) zc[i] -= dot * vs[i];
-    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();  // reflector k is here, k + 1 is no longer read
+    if (k > 0) fetch(k - 1);
+    if (!mine) continue;
+    const double* vs = sm + (k & 1) * (int64_t)max_n;
+    const double tau = S.tau[k];
+    double dot = 0.0;
+    for (int i = k + 1 + lane; i < n; i += 32) dot = fma(vs[i], zc[i], dot);
+    dot = -tau * warp_sum(dot);
+    for (int i = k + 1 + lane; i < n; i += 32) zc[i] = fma(dot, vs[i], zc[i]);
   }
   if (!mine) return;
   const double lam = S.eu[j];
@@ -284,11 +295,11 @@ __global__ void __launch_bounds__(kBtThreads) eig_backtransform(EigBufs b, const
 // Two cluster barriers a column replace two launches of the whole grid.
 // Bound by the FP64 pipe (3 n^3 / 3 FMAs at 1.7 a clock and SM over C SMs)
 // and, per column, by about 40 dependent FP64 operations of 63 clocks each:
-// sums therefore use four warps (one per quarter of the SM), four rows are
-// reduced across a warp's lanes together, and the scalars are formed by one
-// warp.  Measured: see launch_eig_tridiag.
+// sums therefore use four warps (one per quarter of the SM), four rows share
+// a warp's reduction, and the scalars are formed by one warp.  12 matrices up
+// to order 400 in clusters of 16: 2950 us, against 11.7 ms for the tiled
+// launches (17 + 12 us a column).
 constexpr int kClThreads = 512, kClWarps = kClThreads / 32;
-constexpr int kClRows = 4;  // rows per warp at most: C blocks hold 64 C rows
 constexpr int kClSumWarps = 4;
 
 __device__ __forceinline__ void cl_arrive() { __syncwarp(); asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
@@ -398,32 +409,18 @@ __global__ void __launch_bounds__(kClThreads, 1) eig_tridiag_cluster(EigBufs b, 
       if ((uint32_t)i % C == rank) V[(int64_t)k * n + i] = x;
     }
     __syncthreads();
-    // p = A v, the block's rows
-    {
-      double acc[kClRows] = {};
+    // p = A v, the block's rows: eight lanes per row, so that four rows share
+    // a reduction of three steps
+    for (int g = r1 + 4 * warp; g < rows; g += 4 * kClWarps) {
+      const int r = g + (lane >> 3);
+      const bool mine = r < rows;
+      const double* row = a + (mine ? r : g) * ld;
+      double x = 0.0;
+      for (int j = k + 1 + (lane & 7); j < n; j += 8) x = fma(row[j], v[j], x);
 #pragma unroll
-      for (int q = 0; q < kClRows; ++q) {
-        const int r = r1 + warp + kClWarps * q;
-        if (r < rows) {
-          const double* row = a + r * ld;
-          for (int j = k + 1 + lane; j < n; j += 32) acc[q] = fma(row[j], v[j], acc[q]);
-        }
-      }
-      // four sums across the lanes at once: lanes with bit 4 take rows 2, 3,
-      // lanes with bit 3 the odd one of their two
-      if (r1 + warp < rows) {  // warp-uniform
-        const bool hi = lane & 16, odd = lane & 8;
-        double x0 = hi ? acc[2] : acc[0], x1 = hi ? acc[3] : acc[1];
-        x0 += __shfl_xor_sync(0xffffffffu, hi ? acc[0] : acc[2], 16);
-        x1 += __shfl_xor_sync(0xffffffffu, hi ? acc[1] : acc[3], 16);
-        double x = odd ? x1 : x0;
-        x += __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 8);
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        const int r = r1 + warp + kClWarps * ((hi ? 2 : 0) + (odd ? 1 : 0));
-        if (r < rows)
-          for (uint32_t q = lane & 7; q < C; q += 8) cl_store(p + r * (int)C + (int)rank, q, x);
-      }
+      for (int o = 4; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+      if (mine)
+        for (uint32_t q = lane & 7; q < C; q += 8) cl_store(p + r * (int)C + (int)rank, q, x);
     }
     cl_arrive();
     cl_wait();
@@ -465,7 +462,7 @@ __global__ void __launch_bounds__(256) canon_signs_kernel(double* V, const int64
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double* v = V + off[q];
   const bool cm = colmajor[q] != 0;
-  for (int j = warp; j < n; j += 8) {
+  for (int j = warp + 8 * blockIdx.y; j < n; j += 8 * gridDim.y) {
     double best = -1.0, val = 0.0;
     int bi = n;
     for (int i = lane; i < n; i += 32) {
@@ -495,9 +492,33 @@ __global__ void __launch_bounds__(256) canon_signs_kernel(double* V, const int64
   }
 }
 
+// Square matrices transposed, 32 x 32 tiles through shared memory.
+__global__ void __launch_bounds__(256) transpose_kernel(const double* __restrict__ a, double* __restrict__ t,
+                                                        const int64_t* __restrict__ off, const int* __restrict__ dims) {
+  __shared__ double tile[32][33];
+  const int n = dims[blockIdx.x], nt = (n + 31) / 32, x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const double* src = a + off[blockIdx.x];
+  double* dst = t + off[blockIdx.x];
+  for (int b = blockIdx.y; b < nt * nt; b += gridDim.y) {
+    const int r0 = 32 * (b / nt), c0 = 32 * (b % nt);
+    for (int i = y; i < 32; i += 8)
+      if (r0 + i < n && c0 + x < n) tile[i][x] = src[(int64_t)(r0 + i) * n + c0 + x];
+    __syncthreads();
+    for (int i = y; i < 32; i += 8)
+      if (c0 + i < n && r0 + x < n) dst[(int64_t)(c0 + i) * n + r0 + x] = tile[x][i];
+    __syncthreads();
+  }
+}
+
+cudaError_t launch_transpose(const double* a, double* t, const int64_t* off, const int* dims, int nmat,
+                             cudaStream_t s) {
+  if (nmat > 0) transpose_kernel<<<dim3(nmat, 32), 256, 0, s>>>(a, t, off, dims);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_canon_signs(double* V, const int64_t* off, const int* dims, const int* colmajor, int nmat,
                                cudaStream_t s) {
-  if (nmat > 0) canon_signs_kernel<<<nmat, 256, 0, s>>>(V, off, dims, colmajor);
+  if (nmat > 0) canon_signs_kernel<<<dim3(nmat, 8), 256, 0, s>>>(V, off, dims, colmajor);
   return cudaGetLastError();
 }
 
@@ -520,7 +541,7 @@ constexpr size_t kClSmemMax = 226 * 1024;
 
 int eig_cluster_max_n() {
   int n = 1;
-  while (cl_smem(n + 1, 16) <= kClSmemMax && (n + 1 + 15) / 16 <= kClRows * kClWarps) ++n;
+  while (cl_smem(n + 1, 16) <= kClSmemMax) ++n;
   return n;
 }
 
@@ -539,7 +560,7 @@ static int eig_cluster_size(const int* dims, int njobs) {
     return *std::max_element(t.begin(), t.end());
   };
   const int n = dims[0];
-  if (cl_smem(n, 8) > kClSmemMax || (n + 7) / 8 > kClRows * kClWarps) return 16;
+  if (cl_smem(n, 8) > kClSmemMax) return 16;
   return makespan(16, 7) < makespan(8, 15) ? 16 : 8;
 }
 
@@ -574,11 +595,10 @@ cudaError_t launch_eig_backtransform(const EigBufs& b, const EigJob* jobs, int n
                                      cudaStream_t s) {
   if (njobs <= 0) return cudaSuccess;
   if (max_n < 1 || max_n > kEigMaxN) return cudaErrorInvalidValue;
-  const int bt_cols = eig_bt_cols(max_n);
-  const size_t smem_bt = (size_t)(1 + bt_cols) * max_n * sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(eig_backtransform, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bt);
+  const size_t smem = (size_t)(2 + kEigBtCols) * max_n * sizeof(double);
+  cudaError_t e = cudaFuncSetAttribute(eig_backtransform, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  eig_backtransform<<<bt_ctas, kBtThreads, smem_bt, s>>>(b, jobs, njobs, bt_cols);
+  eig_backtransform<<<bt_ctas, kBtThreads, smem, s>>>(b, jobs, njobs, max_n);
   return cudaGetLastError();
 }
 

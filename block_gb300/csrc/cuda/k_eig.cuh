@@ -29,7 +29,7 @@ namespace bgpu {
 namespace dev {
 
 constexpr int kEigTile = 64;     // tile edge of the tridiagonalisation update
-constexpr int kEigBtCols = 8;    // eigenvectors per back-transformation CTA
+constexpr int kEigBtCols = 4;    // eigenvectors per back-transformation CTA (one per warp)
 constexpr int kEigMaxN = 4096;   // largest sector (shared-memory bound of the merges and back-transformation)
 
 // One symmetric matrix of the batch.  All offsets are in doubles.
@@ -42,10 +42,8 @@ struct EigJob {
   int64_t s_off;  // work: d, e, tau, unsorted eigenvalues, w (2 n), partial products (2 nt n)
   int32_t n, nt;  // order, tiles per edge
   int32_t tile0;  // first CTA of this job in the update launch
-  int32_t bt0;    // first CTA of this job in the back-transformation launch
+  int32_t bt0;    // first CTA of this job in the back-transformation launch (ascending over its jobs)
 };
-// eigenvectors per back-transformation CTA for a batch whose largest order is max_n
-inline int eig_bt_cols(int max_n) { return max_n > 2048 ? kEigBtCols / 2 : kEigBtCols; }
 // doubles of the per-job scalar work area
 inline int64_t eig_scalar_elems(int n) {
   const int64_t nt = (n + kEigTile - 1) / kEigTile;
@@ -80,6 +78,9 @@ cudaError_t launch_eig_tridiag_cluster(const EigBufs& b, const EigJob* jobs, con
 // engine up to rotations inside degenerate eigenspaces.
 cudaError_t launch_canon_signs(double* V, const int64_t* off, const int* dims, const int* colmajor, int nmat,
                                cudaStream_t s);
+// matrix q of a (order dims[q] at off[q]) transposed into t at the same place
+cudaError_t launch_transpose(const double* a, double* t, const int64_t* off, const int* dims, int nmat,
+                             cudaStream_t s);
 cudaError_t launch_eig_backtransform(const EigBufs& b, const EigJob* jobs, int njobs, int max_n, int bt_ctas,
                                      cudaStream_t s);
 

@@ -209,8 +209,8 @@ __global__ void __launch_bounds__(256) tc_pack_kernel(TcBufs b, const TcPack* __
   }
 }
 
-cudaError_t launch_tc_pack(const TcBufs& b, const TcPack* units, int nunits, cudaStream_t s) {
-  if (nunits > 0) tc_pack_kernel<<<dim3(nunits, pack_split(nunits)), 256, 0, s>>>(b, units);
+cudaError_t launch_tc_pack(const TcBufs& b, const TcPack* units, int nunits, cudaStream_t s, int split) {
+  if (nunits > 0) tc_pack_kernel<<<dim3(nunits, split), 256, 0, s>>>(b, units);
   return cudaGetLastError();
 }
 
@@ -704,8 +704,8 @@ __global__ void __launch_bounds__(256) tc_reduce_kernel(const float2* __restrict
 }
 
 cudaError_t launch_tc_reduce(const TcBufs& b, const TcTile* tiles, const int64_t* slots, int ntiles, double* sigma,
-                             cudaStream_t s) {
-  if (ntiles > 0) tc_reduce_kernel<<<dim3(ntiles, 32), 256, 0, s>>>(b.partials, tiles, slots, sigma);
+                             cudaStream_t s, int split) {
+  if (ntiles > 0) tc_reduce_kernel<<<dim3(ntiles, split), 256, 0, s>>>(b.partials, tiles, slots, sigma);
   return cudaGetLastError();
 }
 

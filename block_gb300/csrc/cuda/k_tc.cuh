@@ -152,12 +152,16 @@ struct TcBufs {
   int fp16;     // slices are fp16 (else bf16)
 };
 
-// Blocks per unit of the packing launches: the operators of a superblock are
-// tens of thousands of units, four blocks each fill the GPU; psi is a few
-// dozen sectors of up to a million elements, which four blocks each left to
-// 2 % of the threads (18 orbitals, M=1000: 289 us for 40 MB).
-inline int pack_split(int nunits) { return nunits >= 1024 ? 4 : nunits > 64 ? 4096 / nunits : 64; }
-cudaError_t launch_tc_pack(const TcBufs& b, const TcPack* units, int nunits, cudaStream_t s);
+// Blocks per unit of a launch over units of at most `elems` elements (eight
+// of which a thread packs at a time): psi is a few dozen sectors of up to a
+// million elements, which four blocks each left to 2 % of the threads (18
+// orbitals, M=1000: 289 us for 40 MB), while 64 blocks for every unit of a
+// small superblock cost more than they do.
+inline int unit_split(int64_t elems, int per_thread) {
+  const int64_t b = (elems + 256 * per_thread - 1) / (256 * per_thread);
+  return b < 1 ? 1 : b > 64 ? 64 : (int)b;
+}
+cudaError_t launch_tc_pack(const TcBufs& b, const TcPack* units, int nunits, cudaStream_t s, int split = 4);
 // phase 1 or 2 on nblocks persistent blocks: block j runs the work records
 // work[ranges[j].x .. ranges[j].y); nb = output-tile width (kTcRowsB or
 // kTcRowsBWide, the row tile of the B-role pools); limit_ns bounds every
@@ -178,8 +182,9 @@ cudaError_t launch_tc_sigma_pairs(const TcBufs& b, const TcWork* work, const int
 // on an mbarrier that nothing arrives at; out[0] = 1 when the wait gave up,
 // out[1] = nanoseconds waited; *status is set by the wait.
 cudaError_t launch_tc_wait_selftest(int* status, unsigned long long* out, uint64_t limit_ns, cudaStream_t s);
+// split: blocks per tile
 cudaError_t launch_tc_reduce(const TcBufs& b, const TcTile* tiles, const int64_t* slots, int ntiles, double* sigma,
-                             cudaStream_t s);
+                             cudaStream_t s, int split);
 
 // ---------------------------------------------------------------- exact
 //
@@ -232,9 +237,9 @@ static_assert(sizeof(TcxWork) == 80, "TcxWork is 80 bytes");
 
 // row exponents of the units' rows (not needed for units whose exponents
 // the phase-1 kernel has already reduced)
-cudaError_t launch_tcx_rowexp(const TcxBufs& b, const TcPack* units, int nunits, cudaStream_t s);
+cudaError_t launch_tcx_rowexp(const TcxBufs& b, const TcPack* units, int nunits, cudaStream_t s, int split = 1);
 // digit slices of the units
-cudaError_t launch_tcx_pack(const TcxBufs& b, const TcPack* units, int nunits, cudaStream_t s);
+cudaError_t launch_tcx_pack(const TcxBufs& b, const TcPack* units, int nunits, cudaStream_t s, int split = 4);
 // phase 1: T tiles (FP64) and the largest exponent of every T row
 // (atomicMax into ex[kTcPoolS], which must start at kTcxNoExp); phase 2:
 // sigma tiles or FP64 partial tiles
@@ -242,7 +247,7 @@ cudaError_t launch_tcx_sigma(int phase, const TcxBufs& b, const TcxWork* work, c
                              double* sigma, uint64_t limit_ns, cudaStream_t s);
 int tcx_blocks_per_sm();
 cudaError_t launch_tcx_reduce(const TcxBufs& b, const TcTile* tiles, const int64_t* slots, int ntiles, double* sigma,
-                              cudaStream_t s);
+                              cudaStream_t s, int split);
 // every element of x (n ints) = v
 cudaError_t launch_fill_int(int* x, int64_t n, int v, cudaStream_t s);
 

@@ -490,13 +490,13 @@ __global__ void fill_int_kernel(int* x, int64_t n, int v) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) x[i] = v;
 }
 
-cudaError_t launch_tcx_rowexp(const TcxBufs& b, const TcPack* units, int nunits, cudaStream_t s) {
-  if (nunits > 0) tcx_rowexp_kernel<<<dim3(nunits, nunits >= 1024 ? 1 : 8), 256, 0, s>>>(b, units);
+cudaError_t launch_tcx_rowexp(const TcxBufs& b, const TcPack* units, int nunits, cudaStream_t s, int split) {
+  if (nunits > 0) tcx_rowexp_kernel<<<dim3(nunits, split), 256, 0, s>>>(b, units);
   return cudaGetLastError();
 }
 
-cudaError_t launch_tcx_pack(const TcxBufs& b, const TcPack* units, int nunits, cudaStream_t s) {
-  if (nunits > 0) tcx_pack_kernel<<<dim3(nunits, pack_split(nunits)), 256, 0, s>>>(b, units);
+cudaError_t launch_tcx_pack(const TcxBufs& b, const TcPack* units, int nunits, cudaStream_t s, int split) {
+  if (nunits > 0) tcx_pack_kernel<<<dim3(nunits, split), 256, 0, s>>>(b, units);
   return cudaGetLastError();
 }
 
@@ -520,8 +520,8 @@ cudaError_t launch_tcx_sigma(int phase, const TcxBufs& b, const TcxWork* work, c
 int tcx_blocks_per_sm() { return 1; }
 
 cudaError_t launch_tcx_reduce(const TcxBufs& b, const TcTile* tiles, const int64_t* slots, int ntiles, double* sigma,
-                              cudaStream_t s) {
-  if (ntiles > 0) tcx_reduce_kernel<<<dim3(ntiles, 32), 256, 0, s>>>(b.partials, tiles, slots, sigma);
+                              cudaStream_t s, int split) {
+  if (ntiles > 0) tcx_reduce_kernel<<<dim3(ntiles, split), 256, 0, s>>>(b.partials, tiles, slots, sigma);
   return cudaGetLastError();
 }
 

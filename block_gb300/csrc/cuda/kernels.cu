@@ -40,7 +40,7 @@ static_assert(kGK == kGT, "a slab edge is one warp's lanes");
 
 __global__ void __launch_bounds__(kGThreads, 7) gemm_fp64_kernel(Bufs bufs, const GemmUnit* __restrict__ units,
                                                                  const GemmItem* __restrict__ items,
-                                                                 const GemmTask* __restrict__ tasks) {
+                                                                 const GemmTask* __restrict__ tasks, int edge) {
   __shared__ double As[kGK][kGT + 1];
   __shared__ double Bs[kGK][kGT + 1];
   __shared__ GemmItem its[kGItems];
@@ -52,8 +52,8 @@ __global__ void __launch_bounds__(kGThreads, 7) gemm_fp64_kernel(Bufs bufs, cons
 #pragma unroll
     for (int i = 0; i < kMaxBufs; ++i) bp[i] = bufs.p[i];
   }
-  // equal edges (none empty: 32 tiles hold over 31 x 32 rows, more have edge 32)
-  const int nth = (u.m + kGT - 1) / kGT, ntw = (u.n + kGT - 1) / kGT;
+  // equal edges (none empty: n tiles of edge t <= edge hold more than (n - 1) t rows)
+  const int nth = (u.m + edge - 1) / edge, ntw = (u.n + edge - 1) / edge;
   const int th = (u.m + nth - 1) / nth, tw = (u.n + ntw - 1) / ntw;
   const int row0 = task.tm * th, col0 = task.tn * tw;
   const int h = min(th, u.m - row0), w = min(tw, u.n - col0);
@@ -164,9 +164,10 @@ __global__ void __launch_bounds__(kGThreads, 7) gemm_fp64_kernel(Bufs bufs, cons
 }
 
 cudaError_t launch_gemm(const Bufs& bufs, const GemmUnit* units, const GemmItem* items, const GemmTask* tasks,
-                        int ntasks, cudaStream_t s) {
+                        int ntasks, cudaStream_t s, int edge) {
   if (ntasks <= 0) return cudaSuccess;
-  gemm_fp64_kernel<<<ntasks, kGThreads, 0, s>>>(bufs, units, items, tasks);
+  if (edge < 1 || edge > kGemmTile) return cudaErrorInvalidValue;
+  gemm_fp64_kernel<<<ntasks, kGThreads, 0, s>>>(bufs, units, items, tasks, edge);
   return cudaGetLastError();
 }
 

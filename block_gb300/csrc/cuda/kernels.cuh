@@ -45,7 +45,8 @@ struct GemmTask {
   int32_t unit;
   int32_t tm, tn;  // tile indices
 };
-constexpr int kGemmTile = 32;  // output-tile edge of the grouped GEMM
+constexpr int kGemmTile = 32;  // largest output-tile edge of the grouped GEMM
+constexpr int kGemmTileSmall = 16;  // edge for lists that leave SMs idle with kGemmTile
 constexpr int kDiagTile = 64;  // and of the diagonal tiles
 
 // dst rectangle (m x n at c_off, ldc) = sum of items [ibeg, iend)
@@ -79,8 +80,9 @@ struct DiagItem {
 };
 
 // launch helpers (return cudaGetLastError())
+// edge: the tile edge the tasks were made for (at most kGemmTile)
 cudaError_t launch_gemm(const Bufs& bufs, const GemmUnit* units, const GemmItem* items, const GemmTask* tasks,
-                        int ntasks, cudaStream_t s);
+                        int ntasks, cudaStream_t s, int edge = kGemmTile);
 // split: blocks per unit
 cudaError_t launch_copy(const Bufs& bufs, double* dst, const CopyUnit* units, const CopyItem* items, int nunits,
                         cudaStream_t s, int split = 1);
