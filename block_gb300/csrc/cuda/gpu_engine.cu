@@ -496,6 +496,31 @@ void schedule_waves(const std::vector<double>& cost, int nblocks, std::vector<in
   }
 }
 
+// List assignment: every task, in task order, to the block that is free
+// first, so that neighbouring tasks run at the same time on different
+// blocks; block j runs order[ranges[j].x .. ranges[j].y).
+void schedule_list(const std::vector<double>& cost, int nblocks, std::vector<int>& order, std::vector<int2>& ranges) {
+  const int n = (int)cost.size();
+  order.clear();
+  ranges.clear();
+  if (n == 0) return;
+  nblocks = std::max(1, std::min(nblocks, n));
+  std::vector<std::vector<int>> per(nblocks);
+  std::priority_queue<std::pair<double, int>, std::vector<std::pair<double, int>>, std::greater<>> load;
+  for (int j = 0; j < nblocks; ++j) load.push({0.0, j});
+  for (int i = 0; i < n; ++i) {
+    auto [l, j] = load.top();
+    load.pop();
+    per[j].push_back(i);
+    load.push({l + cost[i], j});
+  }
+  for (auto& v : per) {
+    const int b = (int)order.size();
+    order.insert(order.end(), v.begin(), v.end());
+    ranges.push_back(make_int2(b, (int)order.size()));
+  }
+}
+
 void add_tasks(std::vector<dev::GemmTask>& t, int unit, int m, int n, int tile = dev::kGemmTile) {
   for (int a = 0; a < (m + tile - 1) / tile; ++a)
     for (int b = 0; b < (n + tile - 1) / tile; ++b) t.push_back({unit, a, b});
@@ -1663,9 +1688,11 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
   std::vector<TcTask> t2;
   std::vector<double> c2;
   std::vector<int> sec2;
-  std::vector<int64_t> bundle2;
   std::vector<TcTile> tiles;
   std::vector<int64_t> slots;
+  std::vector<int> breaks;  // per tile: items at which an accumulation group starts anew
+  const int group_items = std::max(1, kn.group);
+  constexpr int kGroupK = 1024;
   int64_t partial_n = 0;
   double total = 0.0;
   for (int s = 0; s < nsec; ++s) {
@@ -1779,17 +1806,65 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
       }
     }
   } else {
+    // Bytes a block streams for an item of a tile, and a fixed part in the same
+    // unit for the item's trip through the pipeline (fitted to the blocks'
+    // active clocks at 24 orbitals, M=500: 860 clocks plus a byte per 1/24
+    // clock; by K times columns alone the slowest block took 1.4 times the
+    // mean).
+    auto stream_cost = [&](const TcItem& it, int ha, int hb) { return 20000.0 + 4.0 * (ha + hb) * it.kp; };
+    // Pieces: every tile of a sector is cut at about the same items, into
+    // pieces of at most a kPieces-th of a block's share.  The pieces are laid
+    // out piece by piece and, within one, tile by tile, and dealt to the blocks
+    // in this order (schedule_list): the tiles of a sector then run side by
+    // side over the same items, and their operands, read by one row and one
+    // column of tiles each, come from L2 (24 orbitals, M=500: phase 2 read
+    // 2.4 GB of its 2.6 GB from memory before).  Sectors with more work first.
+    constexpr double kPieces = 6.0;
+    std::vector<double> sec_cost(nsec, 0.0), sec_tile(nsec, 0.0);
+    double stream_total = 0.0;
     for (int s = 0; s < nsec; ++s) {
+      const auto& S = sb.sectors[s];
+      const int rows_p = tc_round8(S.rows), cols_p = tc_round8(S.cols);
+      for (const TcItem& it : per_sector[s]) sec_tile[s] += stream_cost(it, std::min(128, rows_p), std::min(nb, cols_p));
+      for (int tm = 0; tm < (S.rows + 127) / 128; ++tm)
+        for (int tn = 0; tn < (S.cols + nb - 1) / nb; ++tn)
+          for (const TcItem& it : per_sector[s])
+            sec_cost[s] += stream_cost(it, std::min(128, rows_p - 128 * tm), std::min(nb, cols_p - nb * tn));
+      stream_total += sec_cost[s];
+    }
+    const int nblk = (plan.tcx ? tcx_blocks_per_sm() : tc_blocks_per_sm(nb)) * nsm;
+    const double piece = seq ? 1e300 : std::max(stream_total / (kPieces * nblk), 800000.0);
+    std::vector<int> sec_order(nsec);
+    for (int s = 0; s < nsec; ++s) sec_order[s] = s;
+    if (!seq)
+      std::stable_sort(sec_order.begin(), sec_order.end(), [&](int x, int y) { return sec_cost[x] > sec_cost[y]; });
+    for (int s : sec_order) {
       const auto& S = sb.sectors[s];
       const int ib = (int)i2.size();
       i2.insert(i2.end(), per_sector[s].begin(), per_sector[s].end());
       const int ie = (int)i2.size();
       const int rows_p = tc_round8(S.rows), cols_p = tc_round8(S.cols);
-      for (int tm = 0; tm < (S.rows + 127) / 128; ++tm)
-        for (int tn = 0; tn < (S.cols + nb - 1) / nb; ++tn) {
+      const int ntm = (S.rows + 127) / 128, ntn = (S.cols + nb - 1) / nb;
+      // the sector's cuts, by the work of its first tile
+      std::vector<int> cuts{ib};
+      if (sec_tile[s] > piece && ie - ib > 1) {
+        const double per = sec_tile[s] / std::ceil(sec_tile[s] / piece);
+        double acc = 0.0;
+        for (int x = ib; x < ie; ++x) {
+          if (x > cuts.back() && acc + 1e-9 * per >= per * (double)cuts.size()) cuts.push_back(x);
+          acc += stream_cost(i2[x], std::min(128, rows_p), std::min(nb, cols_p));
+        }
+      }
+      cuts.push_back(ie);
+      // accumulation groups: of items with alpha = 1 (the first n1), broken
+      // at every `chunk` of K times columns
+      int n1 = ib;
+      while (n1 < ie && i2[n1].alpha == 1.0f) ++n1;
+      std::vector<std::vector<TcTask>> pieces(cuts.size() - 1);
+      std::vector<std::vector<double>> costs(cuts.size() - 1);
+      for (int tm = 0; tm < ntm; ++tm)
+        for (int tn = 0; tn < ntn; ++tn) {
           const int ha = std::min(128, rows_p - 128 * tm), hb = std::min(nb, cols_p - nb * tn);
-          double tile_cost = 0.0;
-          for (int x = ib; x < ie; ++x) tile_cost += item_cost(i2[x], hb);
           TcTask t{};
           t.a_rows = rows_p;
           t.b_rows = cols_p;
@@ -1798,18 +1873,39 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
           t.valid_rows = std::min(128, S.rows - 128 * tm);
           t.valid_cols = std::min(nb, S.cols - nb * tn);
           for (int x = ib; x < ie; ++x) mma += 3.0 * 2.0 * 128 * tc_round16(hb) * i2[x].kp;
-          if (tile_cost <= chunk || ie - ib <= 1) {
-            t.ibeg = ib;
-            t.iend = ie;
-            t.direct = 1;
-            t.out_off = S.offset;
-            t.out_kp = S.cols;
-            t2.push_back(t);
-            c2.push_back(tile_cost);
-            sec2.push_back(s);
-            bundle2.push_back(((int64_t)s << 8) | tm);
-            continue;
+          double tile_cost = 0.0;
+          for (int x = ib; x < ie; ++x) tile_cost += item_cost(i2[x], hb);
+          std::vector<int> starts;  // group starts among the first n1 items
+          t.bbeg = (int)breaks.size();
+          if (!plan.tcx && n1 > ib) {
+            if (tile_cost > chunk && ie - ib > 1)
+              for (int x0 = ib; x0 < ie;) {
+                double acc = 0.0;
+                int x1 = x0;
+                while (x1 < ie && (acc < chunk || x1 == x0)) acc += item_cost(i2[x1++], hb);
+                if (x1 < n1) breaks.push_back(x1);
+                x0 = x1;
+              }
+            size_t nbk = t.bbeg;
+            for (int x = ib, gn = 0, gk = 0; x < n1; ++x) {
+              const bool brk = nbk < breaks.size() && breaks[nbk] == x;
+              if (brk) ++nbk;
+              if (gn == 0 || brk || gn >= group_items || gk + i2[x].kp > kGroupK) {
+                starts.push_back(x);
+                gn = gk = 0;
+              }
+              ++gn;
+              gk += i2[x].kp;
+            }
           }
+          t.bend = (int)breaks.size();
+          std::vector<int> at;  // this tile's cuts: the sector's, moved back to a group start
+          for (int x : cuts) {
+            if (x > ib && x < n1 && !plan.tcx) x = *(std::upper_bound(starts.begin(), starts.end(), x) - 1);
+            at.push_back(x);
+          }
+          int np = 0;
+          for (size_t c = 0; c + 1 < at.size(); ++c) np += at[c + 1] > at[c] ? 1 : 0;
           TcTile tl{};
           tl.s_off = S.offset;
           tl.lds = S.cols;
@@ -1819,26 +1915,37 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
           tl.c0 = nb * tn;
           tl.pad = hb;  // row stride of the partial slots
           tl.pbeg = (int)slots.size();
-          int x0 = ib;
-          while (x0 < ie) {
-            double acc = 0.0;
-            int x1 = x0;
-            while (x1 < ie && (acc < chunk || x1 == x0)) acc += item_cost(i2[x1++], hb);
+          for (size_t c = 0; c + 1 < at.size(); ++c) {
+            if (at[c + 1] == at[c] && np > 0) continue;
             TcTask u = t;
-            u.ibeg = x0;
-            u.iend = x1;
-            u.direct = 0;
-            u.out_off = partial_n;
-            slots.push_back(partial_n);
-            partial_n += (int64_t)ha * hb;
-            t2.push_back(u);
-            c2.push_back(acc);
-            sec2.push_back(s);
-            bundle2.push_back(-(int64_t)t2.size());  // pieces of a split tile spread over blocks
-            x0 = x1;
+            u.ibeg = at[c];
+            u.iend = at[c + 1];
+            double cost = 0.0;
+            for (int x = u.ibeg; x < u.iend; ++x) cost += stream_cost(i2[x], ha, hb);
+            if (np <= 1) {
+              u.direct = 1;
+              u.out_off = S.offset;
+              u.out_kp = S.cols;
+            } else {
+              u.direct = 0;
+              u.out_off = partial_n;
+              slots.push_back(partial_n);
+              partial_n += (int64_t)ha * hb;
+            }
+            pieces[c].push_back(u);
+            costs[c].push_back(cost);
+            if (np == 0) break;  // a sector without items: one task that writes zeros
           }
-          tl.pend = (int)slots.size();
-          tiles.push_back(tl);
+          if (np > 1) {
+            tl.pend = (int)slots.size();
+            tiles.push_back(tl);
+          }
+        }
+      for (size_t c = 0; c < pieces.size(); ++c)
+        for (size_t k = 0; k < pieces[c].size(); ++k) {
+          t2.push_back(pieces[c][k]);
+          c2.push_back(costs[c][k]);
+          sec2.push_back(s);
         }
     }
   }
@@ -1883,7 +1990,7 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
     } else if (kn.waves) {
       schedule_waves(c2, bps * nsm, o2, r2);
     } else {
-      schedule_lpt(c2, bundle2, bps * nsm, o2, r2);
+      schedule_list(c2, bps * nsm, o2, r2);
     }
   } else {
     // one block per task, tasks grouped by sector, one launch per group
@@ -1911,8 +2018,6 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
   // flatten every block's tasks into its stream of work records; within a
   // task, runs of items with alpha = 1 form accumulation groups of at most
   // kn.group items and kGroupK summed K (f32 accumulation length)
-  const int group_items = std::max(1, kn.group);
-  constexpr int kGroupK = 1024;
   // blocks are flattened in parallel, each into its own slice of records
   auto flatten = [&](int phase, const std::vector<TcTask>& tasks, const std::vector<TcItem>& items,
                      const std::vector<int>& order, const std::vector<int2>& ranges, std::vector<TcWork>& w,
@@ -1959,7 +2064,9 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
           continue;
         }
         int gn = 0, gk = 0;  // items and K in the open group
+        int nbk = T.bbeg;
         for (int i = T.ibeg; i < T.iend; ++i) {
+          while (nbk < T.bend && breaks[nbk] <= i) ++nbk;
           const TcItem& it = items[i];
           TcWork x = base;
           x.a_base = it.a_off + 2 * (int64_t)kTcRowsA * T.tm * it.kp;
@@ -1973,7 +2080,7 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
           if (gn == 0) f |= kTcGStart;
           ++gn;
           gk += it.kp;
-          const bool next_joins = foldable && i + 1 < T.iend && items[i + 1].alpha == 1.0f && gn < group_items &&
+          const bool next_joins = foldable && !(nbk < T.bend && breaks[nbk] == i + 1) && i + 1 < T.iend && items[i + 1].alpha == 1.0f && gn < group_items &&
                                   gk + items[i + 1].kp <= kGroupK;
           if (!next_joins) {
             f |= kTcGEnd;
@@ -2086,6 +2193,16 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
   plan.tc_slots.release(stream_);
   plan.tc_w1.upload(w1, stream_);
   plan.tc_w2.upload(w2, stream_);
+  auto most = [](const std::vector<TcWork>& w) {
+    int2 m = make_int2(16, 16);
+    for (const TcWork& x : w) {
+      m.x = std::max(m.x, x.h_a + x.h_b);
+      m.y = std::max(m.y, x.kp);
+    }
+    return m;
+  };
+  plan.tc_most[0] = most(w1);
+  plan.tc_most[1] = most(w2);
   plan.tc_r1.upload(wr1, stream_);
   plan.tc_r2.upload(wr2, stream_);
   plan.tc_tiles.upload(tiles, stream_);
@@ -2279,19 +2396,19 @@ void GpuEngine::sigma_tc(const Superblock& sb, SigmaPlan& p, const double* psi, 
     // baseline: one launch per psi sector (phase 1) and per sigma sector
     // (phase 2), one block per task
     for (const int2& g : p.tc_l1)
-      cuda_check(dev::launch_tc_sigma(1, p.tc_nb, b, p.tc_w1.d, p.tc_r1.d + g.x, g.y, out, kWaitLimitNs, stream_),
+      cuda_check(dev::launch_tc_sigma(1, p.tc_nb, b, p.tc_w1.d, p.tc_r1.d + g.x, g.y, out, kWaitLimitNs, stream_, p.tc_most[0]),
                  "tc phase 1");
     for (const int2& g : p.tc_l2)
-      cuda_check(dev::launch_tc_sigma(2, p.tc_nb, b, p.tc_w2.d, p.tc_r2.d + g.x, g.y, out, kWaitLimitNs, stream_),
+      cuda_check(dev::launch_tc_sigma(2, p.tc_nb, b, p.tc_w2.d, p.tc_r2.d + g.x, g.y, out, kWaitLimitNs, stream_, p.tc_most[1]),
                  "tc phase 2");
   } else {
-    cuda_check(dev::launch_tc_sigma(1, p.tc_nb, b, p.tc_w1.d, p.tc_r1.d, (int)p.tc_r1.n, out, kWaitLimitNs, stream_),
+    cuda_check(dev::launch_tc_sigma(1, p.tc_nb, b, p.tc_w1.d, p.tc_r1.d, (int)p.tc_r1.n, out, kWaitLimitNs, stream_, p.tc_most[0]),
                "tc phase 1");
     if (p.tc_pairs)
-      cuda_check(dev::launch_tc_sigma_pairs(b, p.tc_w2.d, p.tc_r2.d, (int)p.tc_r2.n, out, kWaitLimitNs, stream_),
+      cuda_check(dev::launch_tc_sigma_pairs(b, p.tc_w2.d, p.tc_r2.d, (int)p.tc_r2.n, out, kWaitLimitNs, stream_, p.tc_most[1]),
                  "tc phase 2 (cluster pairs)");
     else
-      cuda_check(dev::launch_tc_sigma(2, p.tc_nb, b, p.tc_w2.d, p.tc_r2.d, (int)p.tc_r2.n, out, kWaitLimitNs, stream_),
+      cuda_check(dev::launch_tc_sigma(2, p.tc_nb, b, p.tc_w2.d, p.tc_r2.d, (int)p.tc_r2.n, out, kWaitLimitNs, stream_, p.tc_most[1]),
                  "tc phase 2");
   }
   if (marks) cuda_check(cudaEventRecord(marks[1], stream_), "record");

@@ -118,6 +118,7 @@ struct SigmaPlan {
   DevArray<dev::TcPack> tc_psi_pack;
   int tc_psi_split = 1, tc_tile_split = 1;  // blocks per unit of the psi packing and per tile of the partial sums
   DevArray<dev::TcWork> tc_w1, tc_w2;  // work records of phases 1 and 2, grouped by block
+  int2 tc_most[2] = {};                // most rows (A and B together) and K of a record
   DevArray<int2> tc_r1, tc_r2;         // per persistent block: its range of records
   DevArray<dev::TcTile> tc_tiles;
   DevArray<int64_t> tc_slots;

@@ -1,5 +1,7 @@
 // tcgen05 building blocks: a single-tile GEMM used to check the operand
 // layout, descriptors and TMEM read-back against a host product.
+#include <algorithm>
+
 #include "k_tc.cuh"
 #include "tc.cuh"
 
@@ -217,33 +219,37 @@ cudaError_t launch_tc_pack(const TcBufs& b, const TcPack* units, int nunits, cud
 namespace {
 
 // Pipeline shape by output-tile width NB (the B operands' row tile): with
-// NB = 64 two independent blocks share an SM (256 TMEM columns and a
-// 4-stage ring each); with NB = 128 one block owns the SM (512 TMEM
-// columns, a 6-stage ring of 32 KB stages).  One stage holds the largest
-// piece: A (128 rows) and B (NB rows) x 32 columns, hi and lo.
+// NB = 64 two independent blocks share an SM (256 TMEM columns and half the
+// shared memory each); with NB = 128 one block owns the SM.  The ring holds as
+// many stages as fit for the plan's largest piece (tc_ring).
+// Epilogue: one warp per 32 rows and 64 columns.
 template <int NB>
 struct TcCfg {
-  static constexpr int kSlots = NB == 64 ? 4 : 6;
-  static constexpr uint32_t kStageBytes = 2u * (kTcRowsA + NB) * kTcKC * 2;
-  static constexpr int kSmem = kSlots * (int)kStageBytes;
-  static constexpr uint32_t kTmemCols = 4 * NB;     // two accumulators, then the (hi, lo) sums
-  static constexpr uint32_t kVh = 2 * NB, kVl = 3 * NB;
+  static constexpr int kRing = (NB == 64 ? 4 : 6) * 2 * (kTcRowsA + NB) * kTcKC * 2;
+  // an MMA reads 128 rows of A and a multiple of 16 of B, also of a shorter piece
+  static constexpr int kSmem = kRing + 128 * 16 + 16 * 16;
+  static constexpr int kEpiWarps = NB / 16;
+  static constexpr int kThreads = 32 * (kEpiWarps + 2);
+  static constexpr int kProducer = kEpiWarps, kIssuer = kEpiWarps + 1;
+  static constexpr int kAcc = 4;                     // accumulators of NB TMEM columns
+  static constexpr uint32_t kTmemCols = kAcc * NB;
   static constexpr int kBlocksPerSm = NB == 64 ? 2 : 1;
 };
-constexpr int kTcMaxSlots = 6;
-constexpr int kTcThreads = 192;  // warps 0-3 epilogue, 4 bulk-copy producer, 5 MMA issuer
-constexpr int kTcProducer = 4, kTcIssuer = 5;
-constexpr int kTcAcc = 2;        // accumulators of NB TMEM columns
+constexpr int kTcMaxSlots = 16;
+constexpr int kTcMaxAcc = 4;
 
 struct TcShared {
-  uint64_t full[kTcMaxSlots], empty[kTcMaxSlots], acc_full[kTcAcc], acc_empty[kTcAcc], drain;
+  uint64_t full[kTcMaxSlots], empty[kTcMaxSlots], acc_full[kTcMaxAcc], acc_empty[kTcMaxAcc], drain;
   uint32_t tbase;
   int abort_flag;
 };
 
 // bounded wait that also gives up when another role gave up
 __device__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, uint64_t limit_ns) {
-  if (mbar_try_wait(bar, parity)) return true;
+  // polled without the clock first: a read of the global timer takes about a
+  // microsecond, longer than most waits
+  for (int i = 0; i < kSpinPolls; ++i)
+    if (mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = globaltimer_ns();
   while (!mbar_try_wait(bar, parity)) {
     if (*abort_flag) return false;
@@ -256,70 +262,113 @@ __device__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag
   return true;
 }
 
-// hi + lo += x, with the rounding error of the sum kept in lo (TwoSum)
-__device__ __forceinline__ void two_sum_acc(float& hi, float& lo, float x) {
-  const float s = __fadd_rn(hi, x);
-  const float bp = __fsub_rn(s, hi);
-  const float err = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bp)), __fsub_rn(x, bp));
+// hi + lo += x, with the rounding error of the sum kept in lo (TwoSum), two
+// values at a time
+__device__ __forceinline__ void two_sum_acc(uint64_t& hi, uint64_t& lo, uint64_t x) {
+  const uint64_t s = add2(hi, x);
+  const uint64_t bp = sub2(s, hi);
+  const uint64_t err = add2(sub2(hi, sub2(s, bp)), sub2(x, bp));
   hi = s;
-  lo = __fadd_rn(lo, err);
+  lo = add2(lo, err);
 }
 
 }  // namespace
 
-// A warp's batch of up to 32 work records: lane l holds record base + l.
-struct WorkRegs {
-  int4 q[4];
+// Work records are read straight into registers, the next ones while the
+// present one is processed, and prefetched into L1 ahead of that.  (Records
+// held one per lane and handed out by shuffles cost 130 to 290 clocks a
+// shuffle in the one-thread roles' divergent code: 1000 to 2000 clocks an
+// item, more than its copies and MMAs.)
+constexpr int kWorkAhead = 6;  // records prefetched into L1
+__device__ __forceinline__ void prefetch_work(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+__device__ __forceinline__ int64_t join64(int lo, int hi) {
+  return (int64_t)(((uint64_t)(uint32_t)hi << 32) | (uint32_t)lo);
+}
+// what the producer needs of record i (zeros from end on)
+struct CopyRec {
+  int4 base;  // a_base, b_base
+  int kp, hw, pf;
 };
-__device__ __forceinline__ void load_work(const TcWork* __restrict__ w, int idx, int end, WorkRegs& r) {
-  if (idx < end) {
-    const int4* p = reinterpret_cast<const int4*>(w + idx);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) r.q[i] = __ldg(p + i);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) r.q[i] = make_int4(0, 0, 0, 0);
+__device__ __forceinline__ CopyRec load_copy(const TcWork* __restrict__ w, int i, int end) {
+  CopyRec r{};
+  if (i < end) {
+    const int4* p = reinterpret_cast<const int4*>(w + i);
+    r.base = __ldg(p);
+    r.kp = __ldg(&w[i].kp);
+    r.hw = __ldg(reinterpret_cast<const int*>(p + 2));
+    r.pf = __ldg(reinterpret_cast<const int*>(p + 3));
+    if (i + kWorkAhead < end) prefetch_work(w + i + kWorkAhead);
   }
+  return r;
 }
-__device__ __forceinline__ int64_t shfl64(int lo, int hi, int j) {
-  const uint32_t l = (uint32_t)__shfl_sync(0xffffffffu, lo, j), h = (uint32_t)__shfl_sync(0xffffffffu, hi, j);
-  return (int64_t)(((uint64_t)h << 32) | l);
+// the MMA issuer
+struct MmaRec {
+  int kp, hw, pf;
+};
+__device__ __forceinline__ MmaRec load_mma(const TcWork* __restrict__ w, int i, int end) {
+  MmaRec r{};
+  if (i < end) {
+    const int4* p = reinterpret_cast<const int4*>(w + i);
+    r.kp = __ldg(&w[i].kp);
+    r.hw = __ldg(reinterpret_cast<const int*>(p + 2));
+    r.pf = __ldg(reinterpret_cast<const int*>(p + 3));
+    if (i + kWorkAhead < end) prefetch_work(w + i + kWorkAhead);
+  }
+  return r;
 }
-__device__ __forceinline__ int shfl32(int v, int j) { return __shfl_sync(0xffffffffu, v, j); }
+// the epilogue (every lane reads the same record)
+struct EpiRec {
+  int4 q1, q2;  // out_base, kp, alpha; h_a | h_b << 16, valid rows | columns << 16, out_ld, col0
+  int pf;
+};
+__device__ __forceinline__ EpiRec load_epi(const TcWork* __restrict__ w, int i, int end) {
+  EpiRec r{};
+  if (i < end) {
+    const int4* p = reinterpret_cast<const int4*>(w + i);
+    r.q1 = __ldg(p + 1);
+    r.q2 = __ldg(p + 2);
+    r.pf = __ldg(reinterpret_cast<const int*>(p + 3));
+    if (i + kWorkAhead < end) prefetch_work(w + i + kWorkAhead);
+  }
+  return r;
+}
 
 // Grouped split-precision GEMM over packed operands on tcgen05: per K=16
 // step three MMAs (hi*hi + hi*lo + lo*hi) into an f32 TMEM accumulator of
-// 128 x 64; the items of an accumulation group share the accumulator, eight
+// 128 x NB; the items of an accumulation group share the accumulator, four
 // accumulators rotate between groups.  Operand pieces are streamed by bulk
-// copies through an 8-stage shared-memory ring.  Persistent: block j walks the work records [ranges[j].x,
-// ranges[j].y), each role loading them 32 at a time, and the pipeline runs
-// across task boundaries.  The epilogue folds each group sum into a
-// compensated (hi, lo) f32 pair held in registers.
+// copies through the shared-memory ring.  Persistent: block j walks the work
+// records [ranges[j].x, ranges[j].y), and the pipeline runs across task
+// boundaries; the producer and the MMA issuer are one thread each.
+// The epilogue folds each group sum into a compensated (hi, lo) f32 pair per
+// element.  Most groups of a phase-2 task are single items (a stage-1 product
+// read by several spin couplings keeps its factor), so that the fold, not the
+// MMAs, bounded phase 2: with the pairs in TMEM and four warps it took about
+// 3500 clocks a 128 x 128 item (24 orbitals, M=500: 331 items an SM, 680 us).
+// The pairs now stay in registers, 64 columns a thread, folded two values an
+// instruction.
 template <int PHASE, int NB, bool PAIR = false>
-__global__ void __launch_bounds__(kTcThreads, TcCfg<NB>::kBlocksPerSm)
+__global__ void __launch_bounds__(TcCfg<NB>::kThreads, TcCfg<NB>::kBlocksPerSm)
     tc_sigma_kernel(TcBufs b, const TcWork* __restrict__ work, const int2* __restrict__ ranges,
-                    double* __restrict__ sigma, uint64_t limit_ns) {
+                    double* __restrict__ sigma, uint64_t limit_ns, int slots, uint32_t stage_bytes, int piece_k) {
   using Cfg = TcCfg<NB>;
-  constexpr int kTcSlots = Cfg::kSlots;
-  constexpr uint32_t kTcStageBytes = Cfg::kStageBytes;
-  constexpr uint32_t kTcVh = Cfg::kVh, kTcVl = Cfg::kVl;
+  constexpr int kTcProducer = Cfg::kProducer, kTcIssuer = Cfg::kIssuer, kTcAcc = Cfg::kAcc;
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ TcShared sh;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int2 rg = ranges[blockIdx.x];
-  // TMEM: two accumulators of NB columns, then the phase-2 (hi, lo) sums
   if (warp == kTcIssuer) {
     tmem_alloc(&sh.tbase, Cfg::kTmemCols);
     tmem_relinquish();
   }
   if (tid == 0) {
-    for (int i = 0; i < kTcSlots; ++i) {
+    for (int i = 0; i < slots; ++i) {
       mbar_init(&sh.full[i], 1);
       mbar_init(&sh.empty[i], PAIR ? 2 : 1);  // pairs: released by both blocks' MMAs
     }
     for (int i = 0; i < kTcAcc; ++i) {
       mbar_init(&sh.acc_full[i], 1);
-      mbar_init(&sh.acc_empty[i], 4);
+      mbar_init(&sh.acc_empty[i], Cfg::kEpiWarps);
     }
     mbar_init(&sh.drain, 1);
     sh.abort_flag = 0;
@@ -335,287 +384,325 @@ __global__ void __launch_bounds__(kTcThreads, TcCfg<NB>::kBlocksPerSm)
   volatile int* abort_flag = &sh.abort_flag;
 
   if (warp == kTcProducer) {
-    // ---- producer: lane 0 streams the operand pieces (one K-chunk of one
-    // item: A hi, A lo, B hi, B lo) of every item through the stages
-    uint32_t k = 0;  // pieces issued
-    bool ok = true;
-    for (int base = rg.x; base < rg.y && ok; base += 32) {
-      WorkRegs r;
-      load_work(work, base + lane, rg.y, r);
-      const int cnt = min(32, rg.y - base);
-      for (int j = 0; j < cnt && ok; ++j) {
-        const int64_t a_base = shfl64(r.q[0].x, r.q[0].y, j);
-        const int64_t b_base = shfl64(r.q[0].z, r.q[0].w, j);
-        const int kp = shfl32(r.q[1].z, j);
-        const int hw = shfl32(r.q[2].x, j);
-        const int pf = shfl32(r.q[3].x, j);
-        if (lane == 0 && !((pf >> 16) & kTcEmpty)) {
-          const int h_a = hw & 0xffff, h_b = (hw >> 16) & 0xffff;
-          const __nv_bfloat16* pa = pick(b.pool, pf & 0xff) + a_base;
-          const __nv_bfloat16* pb = pick(b.pool, (pf >> 8) & 0xff) + b_base;
-          const int nck = (kp + kTcKC - 1) / kTcKC;
-          for (int c = 0; c < nck; ++c, ++k) {
-            const int w = min(kTcKC, kp - kTcKC * c);
-            const uint32_t abytes = 2u * h_a * w * 2, bbytes = 2u * h_b * w * 2;
-            const int slot = (int)(k % kTcSlots);
-            if (!tc_wait(&sh.empty[slot], ((k / kTcSlots) & 1u) ^ 1u, abort_flag, b.status, limit_ns)) {
-              ok = false;
-              break;
+    // ---- producer (lane 0): streams the operand pieces (up to piece_k columns
+    // of one item, per K-chunk A hi, A lo, then B hi, B lo) through the stages
+    if (lane == 0) {
+      uint32_t k = 0;  // pieces issued
+      int slot = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      CopyRec n0 = load_copy(work, rg.x, rg.y), n1 = load_copy(work, rg.x + 1, rg.y);
+      for (int i = rg.x; i < rg.y && ok; ++i) {
+        const CopyRec r = n0;
+        n0 = n1;
+        n1 = load_copy(work, i + 2, rg.y);
+        if ((r.pf >> 16) & kTcEmpty) continue;
+        const int h_a = r.hw & 0xffff, h_b = (r.hw >> 16) & 0xffff, kp = r.kp;
+        const uint8_t* pa =
+            reinterpret_cast<const uint8_t*>(pick(b.pool, r.pf & 0xff) + join64(r.base.x, r.base.y));
+        const uint8_t* pb =
+            reinterpret_cast<const uint8_t*>(pick(b.pool, (r.pf >> 8) & 0xff) + join64(r.base.z, r.base.w));
+        for (int k0 = 0; k0 < kp; k0 += piece_k, ++k) {
+          const int w = min(piece_k, kp - k0);  // its K-chunks lie one after another
+          const uint32_t abytes = 4u * h_a * w, bbytes = 4u * h_b * w;
+          if (!tc_wait(&sh.empty[slot], ph ^ 1u, abort_flag, b.status, limit_ns)) {
+            ok = false;
+            break;
+          }
+          uint8_t* dst = smem + (uint32_t)slot * stage_bytes;
+          mbar_expect_tx(&sh.full[slot], abytes + bbytes);
+          if constexpr (PAIR) {
+            // this block's half of the A piece's 8-column groups (hi and
+            // lo slices), into the same stage of both blocks of the pair
+            // (piece_k is one chunk)
+            const int ng = w / 8;
+            const int g0 = rank ? (ng + 1) / 2 : 0, g1 = rank ? ng : (ng + 1) / 2;
+            if (g1 > g0) {
+              const uint32_t slice = (uint32_t)h_a * w * 2;
+              const uint32_t off = (uint32_t)g0 * h_a * 16, len = (uint32_t)(g1 - g0) * h_a * 16;
+              bulk_g2s_mc(dst + off, pa + off, len, &sh.full[slot], (uint16_t)3);
+              bulk_g2s_mc(dst + slice + off, pa + slice + off, len, &sh.full[slot], (uint16_t)3);
             }
-            uint8_t* dst = smem + slot * kTcStageBytes;
-            mbar_expect_tx(&sh.full[slot], abytes + bbytes);
-            if constexpr (PAIR) {
-              // this block's half of the A piece's 8-column groups (hi and
-              // lo slices), into the same stage of both blocks of the pair
-              const int ng = w / 8;
-              const int g0 = rank ? (ng + 1) / 2 : 0, g1 = rank ? ng : (ng + 1) / 2;
-              if (g1 > g0) {
-                const uint32_t slice = (uint32_t)h_a * w * 2;
-                const uint32_t off = (uint32_t)g0 * h_a * 16, len = (uint32_t)(g1 - g0) * h_a * 16;
-                const uint8_t* src = reinterpret_cast<const uint8_t*>(pa + 2 * (int64_t)h_a * kTcKC * c);
-                bulk_g2s_mc(dst + off, src + off, len, &sh.full[slot], (uint16_t)3);
-                bulk_g2s_mc(dst + slice + off, src + slice + off, len, &sh.full[slot], (uint16_t)3);
-              }
-            } else {
-              bulk_g2s(dst, pa + 2 * (int64_t)h_a * kTcKC * c, abytes, &sh.full[slot]);
-            }
-            bulk_g2s(dst + abytes, pb + 2 * (int64_t)h_b * kTcKC * c, bbytes, &sh.full[slot]);
+          } else {
+            bulk_g2s(dst, pa, abytes, &sh.full[slot]);
+          }
+          bulk_g2s(dst + abytes, pb, bbytes, &sh.full[slot]);
+          pa += abytes;
+          pb += bbytes;
+          if (++slot == slots) {
+            slot = 0;
+            ph ^= 1u;
           }
         }
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       }
-    }
-    if (lane == 0 && !ok) {
-      // copies already issued still land in shared memory: wait for them
-      for (uint32_t i = (k > kTcSlots ? k - kTcSlots : 0); i < k; ++i)
-        mbar_wait_bounded(&sh.full[i % kTcSlots], (i / kTcSlots) & 1u, limit_ns);
-    }
-    if (PAIR && lane == 0 && ok) {
-      // the last stages released by both blocks: every multicast copy of
-      // this block has landed in the partner and been read there
-      for (uint32_t i = (k > kTcSlots ? k - kTcSlots : 0); i < k; ++i)
-        tc_wait(&sh.empty[i % kTcSlots], (i / kTcSlots) & 1u, abort_flag, b.status, limit_ns);
+      const uint32_t ns = (uint32_t)slots;
+      if (!ok) {
+        // copies already issued still land in shared memory: wait for them
+        for (uint32_t i = (k > ns ? k - ns : 0); i < k; ++i)
+          mbar_wait_bounded(&sh.full[i % ns], (i / ns) & 1u, limit_ns);
+      } else if (PAIR) {
+        // the last stages released by both blocks: every multicast copy of
+        // this block has landed in the partner and been read there
+        for (uint32_t i = (k > ns ? k - ns : 0); i < k; ++i)
+          tc_wait(&sh.empty[i % ns], (i / ns) & 1u, abort_flag, b.status, limit_ns);
+      }
     }
   } else if (warp == kTcIssuer) {
-    // ---- MMA issuer (lane 0)
-    uint32_t k = 0;
+    // ---- MMA issuer: the whole warp walks the records and one lane issues.
+    // An MMA takes its descriptors from uniform registers: in code that one
+    // lane runs by itself every operand is moved there before every MMA,
+    // about 70 clocks an MMA whatever its width, which bounded both phases
+    // (24 orbitals, M=500: 490 clocks for the six MMAs of a piece).
+    int slot = 0;
+    uint32_t ph = 0;
     int ab = 0;
     uint32_t aph = 0;
-    bool ok = true;
-    for (int base = rg.x; base < rg.y && ok; base += 32) {
-      WorkRegs r;
-      load_work(work, base + lane, rg.y, r);
-      const int cnt = min(32, rg.y - base);
-      for (int j = 0; j < cnt && ok; ++j) {
-        const int kp = shfl32(r.q[1].z, j);
-        const int hw = shfl32(r.q[2].x, j);
-        const int pf = shfl32(r.q[3].x, j);
-        const int flags = (pf >> 16) & 0xff;
-        if (lane == 0 && !(flags & kTcEmpty)) {
-          const int h_a = hw & 0xffff, h_b = (hw >> 16) & 0xffff;
-          const uint32_t idesc = b.fp16 ? idesc_f16(128, (h_b + 15) & ~15) : idesc_bf16(128, (h_b + 15) & ~15);
-          if ((flags & kTcGStart) &&
-              !tc_wait(&sh.acc_empty[ab], aph ^ 1u, abort_flag, b.status, limit_ns))
-            ok = false;
-          if (ok) {
-            fence_after_sync();
-            const uint32_t d = tmem + (uint32_t)ab * (uint32_t)NB;
-            const int nck = (kp + kTcKC - 1) / kTcKC;
-            for (int c = 0; c < nck; ++c, ++k) {
-              const int w = min(kTcKC, kp - kTcKC * c);
-              const uint32_t abytes = 2u * h_a * w * 2;
-              const int slot = (int)(k % kTcSlots);
-              if (!tc_wait(&sh.full[slot], (k / kTcSlots) & 1u, abort_flag, b.status, limit_ns)) {
-                ok = false;
-                break;
-              }
-              fence_after_sync();
-              const uint32_t sa = smem_u32(smem + slot * kTcStageBytes);
-              const uint32_t a_lo = (uint32_t)h_a * w * 2, b0 = abytes, b_lo = abytes + (uint32_t)h_b * w * 2;
-              for (int jj = 0; jj < w / 16; ++jj) {
-                const uint32_t ao = (uint32_t)(32 * jj * h_a), bo = (uint32_t)(32 * jj * h_b);
-                const uint64_t dah = smem_desc(sa + ao, h_a * 16, 128);
-                const uint64_t dal = smem_desc(sa + a_lo + ao, h_a * 16, 128);
-                const uint64_t dbh = smem_desc(sa + b0 + bo, h_b * 16, 128);
-                const uint64_t dbl = smem_desc(sa + b_lo + bo, h_b * 16, 128);
-                const uint32_t acc = ((flags & kTcGStart) && c == 0 && jj == 0) ? 0u : 1u;
-                mma_bf16(d, dah, dbh, idesc, acc);
-                mma_bf16(d, dah, dbl, idesc, 1u);
-                mma_bf16(d, dal, dbh, idesc, 1u);
-              }
-              if (PAIR) mma_commit_mc(&sh.empty[slot], (uint16_t)3);
-              else mma_commit(&sh.empty[slot]);
-            }
-            if (ok && (flags & kTcGEnd)) {
-              mma_commit(&sh.acc_full[ab]);
-              if (++ab == kTcAcc) {
-                ab = 0;
-                aph ^= 1u;
-              }
-            }
+    const uint32_t sm0 = smem_u32(smem) >> 4, stage16 = stage_bytes >> 4;
+    const uint32_t idesc0 = b.fp16 ? idesc_f16(128, 0) : idesc_bf16(128, 0);
+    // low words of the operands' descriptors: address / 16 and rows (the
+    // leading byte offset / 16); the high word is the same for all
+    constexpr uint64_t kDescHi = smem_desc_hi();
+    // One piece per step.  The next piece's record and the state of its barrier
+    // are looked at behind the first three MMAs of this one: the queue of the
+    // tensor core is short, and what is done with it empty costs twice.
+    MmaRec n0 = load_mma(work, rg.x, rg.y), n1 = load_mma(work, rg.x + 1, rg.y);
+    int i = rg.x, kp = 0, k0 = 0, flags = 0;
+    uint32_t h_a = 0, h_b = 0, idesc = 0;
+    bool ready = false;
+    auto next_item = [&]() {  // false at the end of the records
+      do {
+        if (i >= rg.y) return false;
+        const int pf = uniform(n0.pf), hw = uniform(n0.hw);
+        kp = uniform(n0.kp);
+        n0 = n1;
+        n1 = load_mma(work, i + 2, rg.y);
+        ++i;
+        flags = (pf >> 16) & 0xff;
+        h_a = (uint32_t)hw & 0xffffu;
+        h_b = (uint32_t)hw >> 16;
+      } while (flags & kTcEmpty);
+      idesc = idesc0 | ((((h_b + 15u) & ~15u) >> 3) << 17);
+      k0 = 0;
+      return true;
+    };
+    bool more = next_item();
+    while (more) {
+      if (k0 == 0 && (flags & kTcGStart) &&
+          !__all_sync(0xffffffffu, tc_wait(&sh.acc_empty[ab], aph ^ 1u, abort_flag, b.status, limit_ns)))
+        break;
+      if (!ready && !__all_sync(0xffffffffu, tc_wait(&sh.full[slot], ph, abort_flag, b.status, limit_ns))) break;
+      fence_after_sync();
+      const uint32_t a0 = sm0 + (uint32_t)slot * stage16;
+      const int w = min(piece_k, kp - k0);
+      const uint32_t b0 = a0 + (h_a * (uint32_t)w >> 2);  // 16-byte units
+      const uint32_t d = tmem + (uint32_t)ab * (uint32_t)NB;
+      const uint32_t idesc_c = idesc, ha = h_a, hb = h_b;
+      const bool gend = (flags & kTcGEnd) && k0 + w >= kp;
+      const uint32_t acc0 = (k0 == 0 && (flags & kTcGStart)) ? 0u : 1u;
+      const int slot_c = slot, ab_c = ab;
+      const uint32_t la = a0 | (ha << 16), lb = b0 | (hb << 16);
+      const int w0 = min(kTcKC, w);
+      // a slice of h rows x w0 columns is h w0 / 8 units
+      const uint64_t dah = kDescHi | la, dal = kDescHi | (la + (ha * (uint32_t)w0 >> 3));
+      const uint64_t dbh = kDescHi | lb, dbl = kDescHi | (lb + (hb * (uint32_t)w0 >> 3));
+      if (elect_one()) {
+        mma_bf16(d, dah, dbh, idesc_c, acc0);
+        mma_bf16(d, dah, dbl, idesc_c, 1u);
+        mma_bf16(d, dal, dbh, idesc_c, 1u);
+      }
+      __syncwarp();
+      if (++slot == slots) {
+        slot = 0;
+        ph ^= 1u;
+      }
+      const bool probe = mbar_test(&sh.full[slot], ph);
+      if (gend && ++ab == kTcAcc) {
+        ab = 0;
+        aph ^= 1u;
+      }
+      k0 += w;
+      if (k0 >= kp) more = next_item();
+      if (elect_one()) {
+        const uint64_t sa = 2 * ha, sb = 2 * hb;  // one K=16 step
+        if (w0 == kTcKC) {
+          mma_bf16(d, dah + sa, dbh + sb, idesc_c, 1u);
+          mma_bf16(d, dah + sa, dbl + sb, idesc_c, 1u);
+          mma_bf16(d, dal + sa, dbh + sb, idesc_c, 1u);
+        }
+        if (w > kTcKC) {  // the second chunk
+          const uint32_t w1 = (uint32_t)w - kTcKC;
+          const uint64_t eah = dah + 8 * ha, eal = eah + (ha * w1 >> 3);
+          const uint64_t ebh = dbh + 8 * hb, ebl = ebh + (hb * w1 >> 3);
+          mma_bf16(d, eah, ebh, idesc_c, 1u);
+          mma_bf16(d, eah, ebl, idesc_c, 1u);
+          mma_bf16(d, eal, ebh, idesc_c, 1u);
+          if (w1 == kTcKC) {
+            mma_bf16(d, eah + sa, ebh + sb, idesc_c, 1u);
+            mma_bf16(d, eah + sa, ebl + sb, idesc_c, 1u);
+            mma_bf16(d, eal + sa, ebh + sb, idesc_c, 1u);
           }
         }
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+        if (PAIR) mma_commit_mc(&sh.empty[slot_c], (uint16_t)3);
+        else mma_commit(&sh.empty[slot_c]);
+        if (gend) mma_commit(&sh.acc_full[ab_c]);
       }
+      __syncwarp();
+      ready = __all_sync(0xffffffffu, probe);
     }
   } else {
-    // ---- epilogue: warp w owns TMEM lanes 32 w.., all NB columns, read in
-    // halves of 64 columns
-    const int row = 32 * warp + lane;
-    const uint32_t lane_base = (uint32_t)(32 * warp) << 16;
-    const uint32_t vh_t = tmem + kTcVh + lane_base, vl_t = tmem + kTcVl + lane_base;
+    // ---- epilogue: warp w reads TMEM lanes 32 (w % 4).., columns
+    // 64 (w / 4)..; thread `row` holds the sums of its row's 64 columns, two
+    // to a register pair
+    const int row = 32 * (warp & 3) + lane;
+    const int cw = 64 * (warp >> 2);  // first column of this warp
+    const uint32_t lane_base = ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)cw;
     int ab = 0;
     uint32_t aph = 0;
     bool ok = true, first = true;
-    for (int base = rg.x; base < rg.y && ok; base += 32) {
-      WorkRegs r;
-      load_work(work, base + lane, rg.y, r);
-      const int cnt = min(32, rg.y - base);
-      for (int j = 0; j < cnt && ok; ++j) {
-        const int pf = shfl32(r.q[3].x, j);
-        const int flags = (pf >> 16) & 0xff;
-        if (!(flags & (kTcFirst | kTcLast | kTcGEnd))) continue;
-        const float alpha = __int_as_float(shfl32(r.q[1].w, j));
-        const int hw = shfl32(r.q[2].x, j);
-        const int h_a = hw & 0xffff, h_b = (hw >> 16) & 0xffff;
-        const int ng = ((h_b + 15) & ~15) >> 4;  // 16-column groups of the accumulator
-        const int64_t out_base = shfl64(r.q[1].x, r.q[1].y, j);
-        const int vrc = shfl32(r.q[2].y, j);
-        const int out_ld = shfl32(r.q[2].z, j);
-        const int col0 = shfl32(r.q[2].w, j);
-        if (flags & kTcFirst) first = true;
-        const bool have = (flags & kTcGEnd) && !(flags & kTcEmpty);
-        const bool last = (flags & kTcLast) != 0;
-        // phase 1: the stage-1 operand, row and scale this thread's row goes to
+    uint64_t vh[PHASE == 2 ? 32 : 1], vl[PHASE == 2 ? 32 : 1];
+    EpiRec nx = load_epi(work, rg.x, rg.y);
+    for (int i = rg.x; i < rg.y && ok; ++i) {
+      const EpiRec r = nx;
+      nx = load_epi(work, i + 1, rg.y);
+      const int flags = (r.pf >> 16) & 0xff;
+      if (!(flags & (kTcFirst | kTcLast | kTcGEnd))) continue;
+      const float alpha = __int_as_float(r.q1.w);
+      const int hw = r.q2.x;
+      const int h_a = hw & 0xffff, h_b = (hw >> 16) & 0xffff;
+      // 16-column groups of the accumulator in this warp's columns
+      const int ng = min(max((((h_b + 15) & ~15) - cw) >> 4, 0), 4);
+      if (flags & kTcFirst) first = true;
+      const bool have = (flags & kTcGEnd) && !(flags & kTcEmpty);
+      const bool last = (flags & kTcLast) != 0;
+      const uint32_t d = tmem + (uint32_t)ab * (uint32_t)NB + lane_base;
+      if (have) {
+        ok = __all_sync(0xffffffffu, tc_wait(&sh.acc_full[ab], aph, abort_flag, b.status, limit_ns));
+        if (!ok) break;  // TMEM loads below need the whole warp
+        fence_after_sync();
+      }
+      if constexpr (PHASE == 2) {
+        if (have) {
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            if (g < ng) {
+              float v[16];
+              tmem_ld16(d + 16u * (uint32_t)g, v);
+              if (g == ng - 1) {
+                // accumulator read: the MMA issuer may reuse it
+                fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sh.acc_empty[ab]);
+              }
+              if (first) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                  vh[8 * g + e] = scale2(alpha, v[2 * e], v[2 * e + 1]);
+                  vl[8 * g + e] = 0ull;
+                }
+              } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                  two_sum_acc(vh[8 * g + e], vl[8 * g + e], scale2(alpha, v[2 * e], v[2 * e + 1]));
+              }
+            }
+          }
+          if (ng == 0 && lane == 0) mbar_arrive(&sh.acc_empty[ab]);
+        } else if (first) {  // a task without items writes zeros
+#pragma unroll
+          for (int e = 0; e < 32; ++e) vh[e] = vl[e] = 0ull;
+        }
+        if (last && !(PAIR && (flags & kTcGhost))) {
+          const int64_t out_base = join64(r.q1.x, r.q1.y);
+          const int vrc = r.q2.y, out_ld = r.q2.z;
+          const bool direct = (flags & kTcDirect) != 0;
+          const int rows = direct ? vrc & 0xffff : h_a;
+          const int cols = (direct ? (vrc >> 16) & 0xffff : h_b) - cw;
+          if (row < rows) {
+            double* out = sigma + out_base + (int64_t)row * out_ld + cw;
+            float2* outp = b.partials + out_base + (int64_t)row * h_b + cw;
+#pragma unroll
+            for (int e = 0; e < 32; ++e) {
+              if (2 * e < cols) {
+                float h0, h1, l0, l1;
+                unpack2(vh[e], h0, h1);
+                unpack2(vl[e], l0, l1);
+                if (direct) {
+                  out[2 * e] = f32_to_f64(h0) + f32_to_f64(l0);
+                  if (2 * e + 1 < cols) out[2 * e + 1] = f32_to_f64(h1) + f32_to_f64(l1);
+                } else {  // h_b is even
+                  outp[2 * e] = make_float2(h0, l0);
+                  outp[2 * e + 1] = make_float2(h1, l1);
+                }
+              }
+            }
+          }
+        }
+        if (have || last) first = false;
+      } else if (have) {
+        // phase 1: S tile written as a packed operand (rows of this tile,
+        // K columns col0.. of S; row s_row of an s_h-row operand); a
+        // stacked tile's rows go to their members' operands and scales
+        const int64_t out_base = join64(r.q1.x, r.q1.y);
+        const int out_ld = r.q2.z, col0 = r.q2.w;
         int64_t s_base = out_base;
         int s_h = h_a, s_row = row;
         float s_alpha = alpha;
-        if (PHASE == 1 && (flags & kTcStacked) && have && row < h_a) {
+        if ((flags & kTcStacked) && row < h_a) {
           const int4 e = __ldg(reinterpret_cast<const int4*>(b.rows + out_base + row));
           s_base = (int64_t)(((uint64_t)(uint32_t)e.y << 32) | (uint32_t)e.x);
           s_h = e.z & 0xffff;
           s_row = (e.z >> 16) & 0xffff;
           s_alpha = __int_as_float(e.w);
         }
-        if (have) {
-          ok = __all_sync(0xffffffffu, tc_wait(&sh.acc_full[ab], aph, abort_flag, b.status, limit_ns));
-          if (!ok) break;  // TMEM loads below need the whole warp
-          fence_after_sync();
-        }
-        const uint32_t dacc = tmem + (uint32_t)ab * (uint32_t)NB + lane_base;
-#pragma unroll 1
-        for (int hh = 0; hh < NB / 64; ++hh) {
-          const int ngh = min(max(ng - 4 * hh, 0), 4);  // 16-column groups of this half
-          float v[64];
-          if (have) {
+        const bool mine = row < h_a && s_h > 0;
+        const int ncols = min(NB, out_ld - col0) - cw;  // S columns of this warp (a multiple of 8)
+        __nv_bfloat16* sp = b.pool[kTcPoolS] + s_base;
 #pragma unroll
-            for (int e = 0; e < 64; ++e) v[e] = 0.f;
-            const uint32_t d = dacc + 64u * (uint32_t)hh;
-            if (ngh > 2) {
-              tmem_ld32(d, v);
-              if (ngh == 4) tmem_ld32(d + 32u, v + 32);
-              else tmem_ld16(d + 32u, v + 32);
-            } else if (ngh == 2) {
-              tmem_ld32(d, v);
-            } else if (ngh == 1) {
-              tmem_ld16(d, v);
-            }
-            if (hh == NB / 64 - 1) {
-              // accumulator read: the MMA issuer may reuse it
+        for (int g = 0; g < 4; ++g) {
+          float v[16];
+          if (g < ng) {
+            tmem_ld16(d + 16u * (uint32_t)g, v);
+            if (g == ng - 1) {
               fence_before_sync();
               __syncwarp();
               if (lane == 0) mbar_arrive(&sh.acc_empty[ab]);
             }
           }
-          if (PHASE == 2) {
-            if (!have && !last) continue;
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              if (g < ngh) {
-                const int cb = 64 * hh + 16 * g;  // first column of this group
-                float vh[16], vl[16];
-                if (first) {
+          for (int g8 = 0; g8 < 2; ++g8) {
+            const int c0 = 16 * g + 8 * g8;  // column in this warp's 64
+            if (mine && c0 < ncols) {
+              // columns of the accumulator beyond h_b (a multiple of 8) are
+              // another operand's: zeros
+              const bool zero = cw + c0 >= h_b;
+              uint32_t hw4[4], lw4[4];
 #pragma unroll
-                  for (int e = 0; e < 16; ++e) {
-                    vh[e] = have ? __fmul_rn(alpha, v[16 * g + e]) : 0.f;
-                    vl[e] = 0.f;
-                  }
-                } else {
-                  tmem_ld16x2(vh_t + (uint32_t)cb, vl_t + (uint32_t)cb, vh, vl);
-                  if (have) {
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) two_sum_acc(vh[e], vl[e], __fmul_rn(alpha, v[16 * g + e]));
-                  }
-                }
-                if (!last) {
-                  tmem_st16(vh_t + (uint32_t)cb, vh);
-                  tmem_st16(vl_t + (uint32_t)cb, vl);
-                } else if (PAIR && (flags & kTcGhost)) {
-                  // the partner's tile repeated for the pair: no output
-                } else if (flags & kTcDirect) {
-                  const int vrows = vrc & 0xffff, vcols = (vrc >> 16) & 0xffff;
-                  if (row < vrows) {
-                    double* out = sigma + out_base + (int64_t)row * out_ld;
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) {
-                      const int col = cb + e;
-                      if (col < vcols) out[col] = (double)vh[e] + (double)vl[e];
-                    }
-                  }
-                } else if (row < h_a) {
-                  float2* out = b.partials + out_base + (int64_t)row * h_b;
-#pragma unroll
-                  for (int e = 0; e < 16; ++e) {
-                    const int col = cb + e;
-                    if (col < h_b) out[col] = make_float2(vh[e], vl[e]);
-                  }
-                }
+              for (int e = 0; e < 4; ++e) {
+                const uint64_t x =
+                    zero ? 0ull : scale2(s_alpha, v[8 * g8 + 2 * e], v[8 * g8 + 2 * e + 1]);
+                split16x2(x, b.fp16 != 0, hw4[e], lw4[e]);
               }
-            }
-          } else if (have && row < h_a && s_h > 0) {
-            // phase 1: S tile written as a packed operand (rows of this tile,
-            // K columns col0.. of S; row s_row of an s_h-row operand)
-            const int ncols = min(NB, out_ld - col0);
-            __nv_bfloat16* sp = b.pool[kTcPoolS] + s_base;
-#pragma unroll
-            for (int g8 = 0; g8 < 8; ++g8) {
-              const int c0 = 64 * hh + 8 * g8;
-              if (c0 < ncols) {
-                uint32_t hw4[4], lw4[4];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                  const float x = (c0 + e) < h_b ? __fmul_rn(s_alpha, v[8 * g8 + e]) : 0.f;
-                  uint32_t bh, bl;
-                  split16(x, b.fp16 != 0, bh, bl);
-                  if (e & 1) {
-                    hw4[e >> 1] |= bh << 16;
-                    lw4[e >> 1] |= bl << 16;
-                  } else {
-                    hw4[e >> 1] = bh;
-                    lw4[e >> 1] = bl;
-                  }
-                }
-                const int C = col0 + c0;  // S column
-                const int cc = C / kTcKC, wc = min(kTcKC, out_ld - kTcKC * cc);
-                const int64_t off = 2 * (int64_t)s_h * kTcKC * cc + (kmajor_off(s_row, C % kTcKC, s_h) >> 1);
-                *(uint4*)(sp + off) = make_uint4(hw4[0], hw4[1], hw4[2], hw4[3]);
-                *(uint4*)(sp + off + (int64_t)s_h * wc) = make_uint4(lw4[0], lw4[1], lw4[2], lw4[3]);
-              }
+              const int Cc = col0 + cw + c0;  // S column
+              const int cc = Cc / kTcKC, wc = min(kTcKC, out_ld - kTcKC * cc);
+              const int64_t off = 2 * (int64_t)s_h * kTcKC * cc + (kmajor_off(s_row, Cc % kTcKC, s_h) >> 1);
+              *(uint4*)(sp + off) = make_uint4(hw4[0], hw4[1], hw4[2], hw4[3]);
+              *(uint4*)(sp + off + (int64_t)s_h * wc) = make_uint4(lw4[0], lw4[1], lw4[2], lw4[3]);
             }
           }
         }
-        if (have && ++ab == kTcAcc) {
-          ab = 0;
-          aph ^= 1u;
-        }
-        if (PHASE == 2 && (have || last)) first = false;
+        if (ng == 0 && lane == 0) mbar_arrive(&sh.acc_empty[ab]);
+      }
+      if (have && ++ab == kTcAcc) {
+        ab = 0;
+        aph ^= 1u;
       }
     }
   }
   __syncthreads();
   if (warp == kTcIssuer) {
     // every MMA of this block has completed before TMEM is released
-    if (lane == 0) {
+    __syncwarp();
+    if (elect_one()) {  // the lane that issued them
       mma_commit(&sh.drain);
       mbar_wait_bounded(&sh.drain, 0, limit_ns);
     }
@@ -627,31 +714,53 @@ __global__ void __launch_bounds__(kTcThreads, TcCfg<NB>::kBlocksPerSm)
   if (PAIR) cluster_sync();
 }
 
+// Columns per piece and stages of the ring for pieces of at most rows rows (A
+// and B together) and kp columns: two K-chunks a piece, which halves the
+// barrier round trips, where three stages of them fit (always with 128-column
+// tiles; with 64 for the pieces of small sectors), else one.
+struct TcRing {
+  int piece_k, stage, slots;
+};
+template <int NB>
+static TcRing tc_ring(int rows, int kp, bool pair) {
+  TcRing r;
+  for (r.piece_k = pair ? kTcKC : 2 * kTcKC;; r.piece_k = kTcKC) {
+    r.stage = (4 * rows * std::min(r.piece_k, kp) + 127) / 128 * 128;
+    r.slots = std::min(kTcMaxSlots, TcCfg<NB>::kRing / r.stage);
+    if (r.slots >= 3 || r.piece_k == kTcKC) return r;
+  }
+}
+
 template <int PHASE, int NB>
 static cudaError_t launch_tc_sigma_nb(const TcBufs& b, const TcWork* work, const int2* ranges, int nblocks,
-                                      double* sigma, uint64_t limit_ns, cudaStream_t s) {
+                                      double* sigma, uint64_t limit_ns, cudaStream_t s, int2 most) {
   constexpr int smem = TcCfg<NB>::kSmem;
+  if (most.x <= 0 || most.x > kTcRowsA + NB || most.y <= 0) return cudaErrorInvalidValue;
+  const TcRing r = tc_ring<NB>(most.x, most.y, false);
   cudaError_t e = cudaFuncSetAttribute(tc_sigma_kernel<PHASE, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  tc_sigma_kernel<PHASE, NB><<<nblocks, kTcThreads, smem, s>>>(b, work, ranges, sigma, limit_ns);
+  tc_sigma_kernel<PHASE, NB><<<nblocks, TcCfg<NB>::kThreads, smem, s>>>(b, work, ranges, sigma, limit_ns, r.slots,
+                                                                       (uint32_t)r.stage, r.piece_k);
   return cudaGetLastError();
 }
 
 cudaError_t launch_tc_sigma(int phase, int nb, const TcBufs& b, const TcWork* work, const int2* ranges, int nblocks,
-                            double* sigma, uint64_t limit_ns, cudaStream_t s) {
+                            double* sigma, uint64_t limit_ns, cudaStream_t s, int2 most) {
   if (nblocks <= 0) return cudaGetLastError();
-  if (phase == 1 && nb == 64) return launch_tc_sigma_nb<1, 64>(b, work, ranges, nblocks, sigma, limit_ns, s);
-  if (phase == 2 && nb == 64) return launch_tc_sigma_nb<2, 64>(b, work, ranges, nblocks, sigma, limit_ns, s);
-  if (phase == 1 && nb == 128) return launch_tc_sigma_nb<1, 128>(b, work, ranges, nblocks, sigma, limit_ns, s);
-  if (phase == 2 && nb == 128) return launch_tc_sigma_nb<2, 128>(b, work, ranges, nblocks, sigma, limit_ns, s);
+  if (phase == 1 && nb == 64) return launch_tc_sigma_nb<1, 64>(b, work, ranges, nblocks, sigma, limit_ns, s, most);
+  if (phase == 2 && nb == 64) return launch_tc_sigma_nb<2, 64>(b, work, ranges, nblocks, sigma, limit_ns, s, most);
+  if (phase == 1 && nb == 128) return launch_tc_sigma_nb<1, 128>(b, work, ranges, nblocks, sigma, limit_ns, s, most);
+  if (phase == 2 && nb == 128) return launch_tc_sigma_nb<2, 128>(b, work, ranges, nblocks, sigma, limit_ns, s, most);
   return cudaErrorInvalidValue;
 }
 
 int tc_blocks_per_sm(int nb) { return nb == 64 ? TcCfg<64>::kBlocksPerSm : TcCfg<128>::kBlocksPerSm; }
 
 cudaError_t launch_tc_sigma_pairs(const TcBufs& b, const TcWork* work, const int2* ranges, int nblocks, double* sigma,
-                                  uint64_t limit_ns, cudaStream_t s) {
+                                  uint64_t limit_ns, cudaStream_t s, int2 most) {
   if (nblocks <= 0) return cudaGetLastError();
+  if (most.x <= 0 || most.x > 2 * kTcRowsA || most.y <= 0) return cudaErrorInvalidValue;
+  const TcRing r = tc_ring<128>(most.x, most.y, true);
   if (nblocks % 2) return cudaErrorInvalidValue;
   constexpr int smem = TcCfg<128>::kSmem;
   auto kern = tc_sigma_kernel<2, 128, true>;
@@ -659,7 +768,7 @@ cudaError_t launch_tc_sigma_pairs(const TcBufs& b, const TcWork* work, const int
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nblocks);
-  cfg.blockDim = dim3(kTcThreads);
+  cfg.blockDim = dim3(TcCfg<128>::kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -669,7 +778,7 @@ cudaError_t launch_tc_sigma_pairs(const TcBufs& b, const TcWork* work, const int
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, kern, b, work, ranges, sigma, limit_ns);
+  e = cudaLaunchKernelEx(&cfg, kern, b, work, ranges, sigma, limit_ns, r.slots, (uint32_t)r.stage, r.piece_k);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
@@ -693,11 +802,11 @@ __global__ void __launch_bounds__(256) tc_reduce_kernel(const float2* __restrict
 #pragma unroll
       for (int i = 0; i < 8; ++i) v[i] = src[slots[p + i]];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc += (double)v[i].x + (double)v[i].y;
+      for (int i = 0; i < 8; ++i) acc += f32_to_f64(v[i].x) + f32_to_f64(v[i].y);
     }
     for (; p < t.pend; ++p) {
       const float2 v = src[slots[p]];
-      acc += (double)v.x + (double)v.y;
+      acc += f32_to_f64(v.x) + f32_to_f64(v.y);
     }
     sigma[t.s_off + (int64_t)(t.r0 + r) * t.lds + t.c0 + c] = acc;
   }

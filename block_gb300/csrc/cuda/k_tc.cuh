@@ -91,6 +91,7 @@ struct TcTask {
   int32_t valid_rows, valid_cols;
   int32_t stacked;
   int32_t ghost;  // cluster pairs: repeats its partner's tile, writes nothing
+  int32_t bbeg, bend;  // phase 2: the tile's group breaks in the host plan's list
 };
 
 // Row r of a stacked phase-1 tile: row lrow of the packed stage-1 operand S
@@ -165,9 +166,10 @@ cudaError_t launch_tc_pack(const TcBufs& b, const TcPack* units, int nunits, cud
 // phase 1 or 2 on nblocks persistent blocks: block j runs the work records
 // work[ranges[j].x .. ranges[j].y); nb = output-tile width (kTcRowsB or
 // kTcRowsBWide, the row tile of the B-role pools); limit_ns bounds every
-// pipeline wait
+// pipeline wait; most: the most rows of A and B together and the most K of a
+// record (they size the ring's stages)
 cudaError_t launch_tc_sigma(int phase, int nb, const TcBufs& b, const TcWork* work, const int2* ranges, int nblocks,
-                            double* sigma, uint64_t limit_ns, cudaStream_t s);
+                            double* sigma, uint64_t limit_ns, cudaStream_t s, int2 most);
 // persistent blocks per SM of the kernels with tile width nb
 int tc_blocks_per_sm(int nb);
 // Phase 2 with 128-column tiles on pairs of blocks in thread-block clusters
@@ -177,7 +179,7 @@ int tc_blocks_per_sm(int nb);
 // stages with a cluster-multicast bulk copy and its own B piece, and a stage
 // is refilled once both blocks' MMAs released it.  nblocks is even.
 cudaError_t launch_tc_sigma_pairs(const TcBufs& b, const TcWork* work, const int2* ranges, int nblocks, double* sigma,
-                                  uint64_t limit_ns, cudaStream_t s);
+                                  uint64_t limit_ns, cudaStream_t s, int2 most);
 // Bounded-wait self-check: one thread waits, with the sigma kernels' wait,
 // on an mbarrier that nothing arrives at; out[0] = 1 when the wait gave up,
 // out[1] = nanoseconds waited; *status is set by the wait.

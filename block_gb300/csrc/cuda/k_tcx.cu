@@ -158,7 +158,8 @@ struct TcxShared {
 };
 
 __device__ bool tcx_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, uint64_t limit_ns) {
-  if (mbar_try_wait(bar, parity)) return true;
+  for (int i = 0; i < kSpinPolls; ++i)  // without the clock first (tc_wait)
+    if (mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = globaltimer_ns();
   while (!mbar_try_wait(bar, parity)) {
     if (*abort_flag) return false;

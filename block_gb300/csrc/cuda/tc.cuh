@@ -37,6 +37,10 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
   return d;
 }
 
+// its high word (stride byte offset 128 and the version), in place: the low
+// word is start / 16 | (leading byte offset / 16) << 16
+__host__ __device__ constexpr uint64_t smem_desc_hi() { return ((uint64_t)(128 >> 4) << 32) | ((uint64_t)1 << 46); }
+
 // instruction descriptor of kind::f16 with bf16 A and B (both K-major),
 // f32 accumulator, shape M x N
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
@@ -95,6 +99,17 @@ __device__ __forceinline__ void fence_before_sync() {
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 // generic-proxy shared-memory writes become visible to the tensor core
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// one lane of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+// x of lane 0, known to be the same in every lane
+__device__ __forceinline__ int uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
 
 // D[tmem] (+)= A[smem] * B[smem]^T  (issued by one thread)
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
@@ -172,6 +187,57 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* v) {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+// ---- packed pairs of f32 (one instruction for two values, rounded each) ----
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ void unpack2(uint64_t p, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p));
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// products rounded by themselves: a packed product that only feeds packed
+// sums was contracted with them (the sums of a triplet state then moved by
+// 1.5e-8, the rounding of the products)
+__device__ __forceinline__ uint64_t scale2(float a, float lo, float hi) {
+  return pack2(__fmul_rn(a, lo), __fmul_rn(a, hi));
+}
+// (double)x by integer operations (the conversion takes a slot of the FP64
+// pipe, a sixteenth of the rate)
+__device__ __forceinline__ double f32_to_f64(float x) {
+  const uint32_t u = __float_as_uint(x), e = u & 0x7f800000u;
+  if (e == 0u ? (u & 0x7fffffffu) != 0u : e == 0x7f800000u) return (double)x;  // subnormal, infinite or NaN
+  const uint32_t hi = e ? ((u & 0x7fffffffu) >> 3) + 0x38000000u : 0u;
+  return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)(u << 29));
+}
+// split16 of two values: hi and lo hold the slices of x (low half) and y
+__device__ __forceinline__ void split16x2(uint64_t xy, bool fp16, uint32_t& hi, uint32_t& lo) {
+  float x, y;
+  unpack2(xy, x, y);
+  uint64_t h;
+  if (fp16) {
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(y), "f"(x));
+    h = pack2(__half2float(__ushort_as_half((unsigned short)(hi & 0xffffu))),
+              __half2float(__ushort_as_half((unsigned short)(hi >> 16))));
+  } else {
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(y), "f"(x));
+    h = pack2(__uint_as_float(hi << 16), __uint_as_float(hi & 0xffff0000u));
+  }
+  unpack2(sub2(xy, h), x, y);
+  if (fp16) asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(y), "f"(x));
+  else asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(y), "f"(x));
+}
+
 // ---- mbarrier ----
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -186,6 +252,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// whether the phase has completed, without waiting (try_wait may suspend the thread)
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+constexpr int kSpinPolls = 1000;  // polls of a wait before it looks at the clock
 __device__ __forceinline__ uint64_t globaltimer_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

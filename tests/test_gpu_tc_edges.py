@@ -1,0 +1,67 @@
+"""Tensor-core products at the edges of their tiles and stages: one-sector
+superblocks with 1 to 270 rows and columns (tiles of 128 rows and 64 or 128
+columns, 64 columns per epilogue warp, stages cut to the largest piece), a
+stage-1 product, both identity terms and repeated terms (accumulation groups
+and single items with their own factors), against numpy.
+
+Tolerances, of the 2-norm: 2e-5 for two 16-bit slices (the split products'
+bound of the other tests), 1e-11 for the exact slices."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def superblock(ctx, rows, cols, rng, nterms):
+    keys = np.array([[0, -1, -1, 0], [2, 0, 0, 0]], np.int32)  # HAM, CD(0,0;0): both rank 0
+    hl, n = ctx.block_define([0], "c1", [[1, 1, 0]], [rows], keys)
+    hr, m = ctx.block_define([0], "c1", [[1, 1, 0]], [cols], keys)
+    A, B = rng.standard_normal((2, rows, rows)), rng.standard_normal((2, cols, cols))
+    ctx.block_upload(hl, A.reshape(-1))
+    ctx.block_upload(hr, B.reshape(-1))
+    ops = [(0, 0, -1, 0), (-1, 0, 0, 1)] + [(1, t % 2, 1, t // 2 % 2) for t in range(nterms)]
+    coef = np.concatenate([[1.0, -0.5], rng.uniform(0.5, 1.5, nterms)])
+    sb, size = ctx.superblock_define(hl, hr, [2, 0, 0], coef, np.array(ops, np.int32), 0.25)
+    assert size == rows * cols
+
+    def sigma(psi):
+        out = 0.25 * psi + coef[0] * A[0] @ psi + coef[1] * psi @ B[0]
+        for c, (_, lt, _, rt) in zip(coef[2:], ops[2:]):
+            out += c * (A[1].T if lt else A[1]) @ psi @ (B[1] if rt else B[1].T)
+        return out
+
+    return sb, sigma
+
+
+@pytest.mark.parametrize("width", [64, 128])
+@pytest.mark.parametrize("rows,cols", [(1, 1), (8, 9), (17, 63), (64, 65), (65, 120), (127, 128), (129, 136), (270, 200), (128, 270)])
+def test_split_edges(gpu_ctx, rows, cols, width):
+    rng = np.random.default_rng(1000 * rows + cols)
+    try:
+        gpu_ctx.set_tc_tile_width(width)
+        for nterms in (0, 1, 5, 40):
+            sb, sigma = superblock(gpu_ctx, rows, cols, rng, nterms)
+            for prec in ("bf16x3tc", "fp16x2tc"):
+                gpu_ctx.set_precision(prec)
+                psi = rng.standard_normal((rows, cols))
+                ref = sigma(psi)
+                got = gpu_ctx.sigma(sb, psi.reshape(-1)).reshape(rows, cols)
+                assert np.linalg.norm(got - ref) <= 2e-5 * np.linalg.norm(ref), (nterms, prec)
+    finally:
+        gpu_ctx.set_tc_tile_width(0)
+        gpu_ctx.set_precision("fp64")
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (8, 9), (17, 63), (65, 120), (129, 136), (270, 200)])
+def test_exact_edges(gpu_ctx, rows, cols):
+    rng = np.random.default_rng(1000 * rows + cols)
+    try:
+        gpu_ctx.set_precision("exacttc")
+        for nterms in (0, 1, 5, 40):
+            sb, sigma = superblock(gpu_ctx, rows, cols, rng, nterms)
+            psi = rng.standard_normal((rows, cols))
+            ref = sigma(psi)
+            got = gpu_ctx.sigma(sb, psi.reshape(-1)).reshape(rows, cols)
+            assert np.linalg.norm(got - ref) <= 1e-11 * np.linalg.norm(ref), nterms
+    finally:
+        gpu_ctx.set_precision("fp64")
