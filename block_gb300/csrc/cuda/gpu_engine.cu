@@ -1658,7 +1658,6 @@ TcKnobs GpuEngine::tc_default_knobs() const {
   k.split = env_double("BGPU_TC_SPLIT", 3.0);
   k.group = (int)env_double("BGPU_TC_GROUP", 16.0);
   k.waves = (int)env_double("BGPU_TC_WAVES", 0.0);
-  k.pairs = (int)env_double("BGPU_TC_PAIRS", 0.0);
   return k;
 }
 
@@ -1703,115 +1702,18 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
     }
   }
   const double chunk = seq ? 1e300 : std::max(total / (2.0 * kn.split * nsm), 20000.0);
-  // cluster pairs (phase 2 with 128-column tiles): the column tiles tn and
-  // tn + 1 of a sigma row tile run on the two blocks of a cluster, which
-  // read the same items; a row tile with an odd number of column tiles
-  // pairs its last one with a ghost copy that writes nothing.  Split tiles
-  // cut every column tile of a row tile at the same items.  t2 holds the
-  // pairs' tasks one after the other (2p, 2p + 1), c2 their pair costs.
-  const bool pairs = kn.pairs != 0 && nb == kTcRowsBWide && !seq && !plan.tcx;
-  std::vector<double> cp;  // cost per pair
-  std::vector<int64_t> bundle_p;
-  if (pairs) {
-    for (int s = 0; s < nsec; ++s) {
-      const auto& S = sb.sectors[s];
-      const int ib = (int)i2.size();
-      i2.insert(i2.end(), per_sector[s].begin(), per_sector[s].end());
-      const int ie = (int)i2.size();
-      const int rows_p = tc_round8(S.rows), cols_p = tc_round8(S.cols);
-      const int ntn = (S.cols + nb - 1) / nb;
-      for (int tm = 0; tm < (S.rows + 127) / 128; ++tm) {
-        const int ha = std::min(128, rows_p - 128 * tm);
-        const int hb0 = std::min(nb, cols_p);  // the widest column tile
-        double tile_cost = 0.0;
-        for (int x = ib; x < ie; ++x) tile_cost += item_cost(i2[x], hb0);
-        // item cuts shared by every column tile of this row tile
-        std::vector<int2> cuts;
-        if (tile_cost <= chunk || ie - ib <= 1) {
-          cuts.push_back(make_int2(ib, ie));
-        } else {
-          int x0 = ib;
-          while (x0 < ie) {
-            double acc = 0.0;
-            int x1 = x0;
-            while (x1 < ie && (acc < chunk || x1 == x0)) acc += item_cost(i2[x1++], hb0);
-            cuts.push_back(make_int2(x0, x1));
-            x0 = x1;
-          }
-        }
-        const bool direct = cuts.size() == 1;
-        // per column tile: its tasks (one per cut), partial slots and tile
-        std::vector<std::vector<TcTask>> col(ntn);
-        std::vector<std::vector<double>> colc(ntn);
-        for (int tn = 0; tn < ntn; ++tn) {
-          const int hb = std::min(nb, cols_p - nb * tn);
-          TcTask t{};
-          t.a_rows = rows_p;
-          t.b_rows = cols_p;
-          t.tm = tm;
-          t.tn = tn;
-          t.valid_rows = std::min(128, S.rows - 128 * tm);
-          t.valid_cols = std::min(nb, S.cols - nb * tn);
-          for (int x = ib; x < ie; ++x) mma += 3.0 * 2.0 * 128 * tc_round16(hb) * i2[x].kp;
-          TcTile tl{};
-          if (!direct) {
-            tl.s_off = S.offset;
-            tl.lds = S.cols;
-            tl.h = t.valid_rows;
-            tl.w = t.valid_cols;
-            tl.r0 = 128 * tm;
-            tl.c0 = nb * tn;
-            tl.pad = hb;
-            tl.pbeg = (int)slots.size();
-          }
-          for (const int2& ct : cuts) {
-            TcTask u = t;
-            u.ibeg = ct.x;
-            u.iend = ct.y;
-            double acc = 0.0;
-            for (int x = ct.x; x < ct.y; ++x) acc += item_cost(i2[x], hb);
-            if (direct) {
-              u.direct = 1;
-              u.out_off = S.offset;
-              u.out_kp = S.cols;
-            } else {
-              u.direct = 0;
-              u.out_off = partial_n;
-              slots.push_back(partial_n);
-              partial_n += (int64_t)ha * hb;
-            }
-            col[tn].push_back(u);
-            colc[tn].push_back(acc);
-          }
-          if (!direct) {
-            tl.pend = (int)slots.size();
-            tiles.push_back(tl);
-          }
-        }
-        for (int tn = 0; tn < ntn; tn += 2)
-          for (size_t k = 0; k < cuts.size(); ++k) {
-            const TcTask& a = col[tn][k];
-            TcTask g = a;  // ghost partner of a last odd column tile
-            g.ghost = 1;
-            const TcTask& bt = tn + 1 < ntn ? col[tn + 1][k] : g;
-            t2.push_back(a);
-            t2.push_back(bt);
-            sec2.push_back(s);
-            sec2.push_back(s);
-            c2.push_back(colc[tn][k]);
-            c2.push_back(tn + 1 < ntn ? colc[tn + 1][k] : colc[tn][k]);
-            cp.push_back(std::max(c2[c2.size() - 2], c2.back()));
-            bundle_p.push_back(direct ? (((int64_t)s << 8) | tm) : -(int64_t)cp.size());
-          }
-      }
-    }
-  } else {
-    // Bytes a block streams for an item of a tile, and a fixed part in the same
-    // unit for the item's trip through the pipeline (fitted to the blocks'
-    // active clocks at 24 orbitals, M=500: 860 clocks plus a byte per 1/24
-    // clock; by K times columns alone the slowest block took 1.4 times the
-    // mean).
-    auto stream_cost = [&](const TcItem& it, int ha, int hb) { return 20000.0 + 4.0 * (ha + hb) * it.kp; };
+  {
+    // Clocks of an item of a tile: its MMAs (three per K=16 step, each reading
+    // 128 rows of A and the columns of B from shared memory at 128 bytes a
+    // clock), the trips through the pipeline of the item and of its pieces
+    // of 64 K, and a little for its bytes (fitted to the blocks' clocks at
+    // 24 orbitals M=500 and 18 orbitals M=1000, 1 % rms; by K times columns
+    // alone the slowest block took 1.4 times the mean).
+    // Sums over items of a sector come from prefix sums of what does not
+    // depend on the tile (trips) and of K.
+    const double mma_step = (plan.tcx ? 21.0 : 3.0) / 16.0;
+    auto trips = [](const TcItem& it) { return 140.0 + 250.0 * ((it.kp + 63) / 64); };
+    auto per_k = [&](int ha, int hb) { return mma_step * (32.0 + tc_round16(hb) / 4.0) + 0.016 * (ha + hb); };
     // Pieces: every tile of a sector is cut at about the same items, into
     // pieces of at most a kPieces-th of a block's share.  The pieces are laid
     // out piece by piece and, within one, tile by tile, and dealt to the blocks
@@ -1825,15 +1727,19 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
     for (int s = 0; s < nsec; ++s) {
       const auto& S = sb.sectors[s];
       const int rows_p = tc_round8(S.rows), cols_p = tc_round8(S.cols);
-      for (const TcItem& it : per_sector[s]) sec_tile[s] += stream_cost(it, std::min(128, rows_p), std::min(nb, cols_p));
+      double t = 0.0, k = 0.0;
+      for (const TcItem& it : per_sector[s]) {
+        t += trips(it);
+        k += it.kp;
+      }
+      sec_tile[s] = t + k * per_k(std::min(128, rows_p), std::min(nb, cols_p));
       for (int tm = 0; tm < (S.rows + 127) / 128; ++tm)
         for (int tn = 0; tn < (S.cols + nb - 1) / nb; ++tn)
-          for (const TcItem& it : per_sector[s])
-            sec_cost[s] += stream_cost(it, std::min(128, rows_p - 128 * tm), std::min(nb, cols_p - nb * tn));
+          sec_cost[s] += t + k * per_k(std::min(128, rows_p - 128 * tm), std::min(nb, cols_p - nb * tn));
       stream_total += sec_cost[s];
     }
     const int nblk = (plan.tcx ? tcx_blocks_per_sm() : tc_blocks_per_sm(nb)) * nsm;
-    const double piece = seq ? 1e300 : std::max(stream_total / (kPieces * nblk), 800000.0);
+    const double piece = seq ? 1e300 : std::max(stream_total / (kPieces * nblk), 12000.0);
     std::vector<int> sec_order(nsec);
     for (int s = 0; s < nsec; ++s) sec_order[s] = s;
     if (!seq)
@@ -1845,21 +1751,64 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
       const int ie = (int)i2.size();
       const int rows_p = tc_round8(S.rows), cols_p = tc_round8(S.cols);
       const int ntm = (S.rows + 127) / 128, ntn = (S.cols + nb - 1) / nb;
+      std::vector<double> pt(ie - ib + 1, 0.0), pk(ie - ib + 1, 0.0);
+      for (int x = ib; x < ie; ++x) {
+        pt[x - ib + 1] = pt[x - ib] + trips(i2[x]);
+        pk[x - ib + 1] = pk[x - ib] + i2[x].kp;
+      }
       // the sector's cuts, by the work of its first tile
       std::vector<int> cuts{ib};
       if (sec_tile[s] > piece && ie - ib > 1) {
         const double per = sec_tile[s] / std::ceil(sec_tile[s] / piece);
-        double acc = 0.0;
-        for (int x = ib; x < ie; ++x) {
-          if (x > cuts.back() && acc + 1e-9 * per >= per * (double)cuts.size()) cuts.push_back(x);
-          acc += stream_cost(i2[x], std::min(128, rows_p), std::min(nb, cols_p));
-        }
+        const double ck = per_k(std::min(128, rows_p), std::min(nb, cols_p));
+        for (int x = ib + 1; x < ie; ++x)
+          if (pt[x - ib] + ck * pk[x - ib] + 1e-9 * per >= per * (double)cuts.size()) cuts.push_back(x);
       }
       cuts.push_back(ie);
       // accumulation groups: of items with alpha = 1 (the first n1), broken
       // at every `chunk` of K times columns
       int n1 = ib;
       while (n1 < ie && i2[n1].alpha == 1.0f) ++n1;
+      struct Groups {  // of the tiles of one width
+        int hb, bbeg, bend;
+        std::vector<int> at;  // the sector's cuts moved back to group starts
+      };
+      std::vector<Groups> widths;
+      auto groups_of = [&](int hb) -> const Groups& {
+        for (const Groups& g : widths)
+          if (g.hb == hb) return g;
+        Groups g{hb, (int)breaks.size(), 0, {}};
+        std::vector<int> starts;  // group starts among the first n1 items
+        if (!plan.tcx && n1 > ib) {
+          const double tile_cost = item_fixed * (ie - ib) + pk.back() * tc_round16(hb) / 8.0;
+          if (tile_cost > chunk && ie - ib > 1)
+            for (int x0 = ib; x0 < n1;) {
+              double acc = 0.0;
+              int x1 = x0;
+              while (x1 < ie && (acc < chunk || x1 == x0)) acc += item_cost(i2[x1++], hb);
+              if (x1 < n1) breaks.push_back(x1);
+              x0 = x1;
+            }
+          size_t nbk = g.bbeg;
+          for (int x = ib, gn = 0, gk = 0; x < n1; ++x) {
+            const bool brk = nbk < breaks.size() && breaks[nbk] == x;
+            if (brk) ++nbk;
+            if (gn == 0 || brk || gn >= group_items || gk + i2[x].kp > kGroupK) {
+              starts.push_back(x);
+              gn = gk = 0;
+            }
+            ++gn;
+            gk += i2[x].kp;
+          }
+        }
+        g.bend = (int)breaks.size();
+        for (int x : cuts) {
+          if (x > ib && x < n1 && !plan.tcx) x = *(std::upper_bound(starts.begin(), starts.end(), x) - 1);
+          g.at.push_back(x);
+        }
+        widths.push_back(std::move(g));
+        return widths.back();
+      };
       std::vector<std::vector<TcTask>> pieces(cuts.size() - 1);
       std::vector<std::vector<double>> costs(cuts.size() - 1);
       for (int tm = 0; tm < ntm; ++tm)
@@ -1872,38 +1821,12 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
           t.tn = tn;
           t.valid_rows = std::min(128, S.rows - 128 * tm);
           t.valid_cols = std::min(nb, S.cols - nb * tn);
-          for (int x = ib; x < ie; ++x) mma += 3.0 * 2.0 * 128 * tc_round16(hb) * i2[x].kp;
-          double tile_cost = 0.0;
-          for (int x = ib; x < ie; ++x) tile_cost += item_cost(i2[x], hb);
-          std::vector<int> starts;  // group starts among the first n1 items
-          t.bbeg = (int)breaks.size();
-          if (!plan.tcx && n1 > ib) {
-            if (tile_cost > chunk && ie - ib > 1)
-              for (int x0 = ib; x0 < ie;) {
-                double acc = 0.0;
-                int x1 = x0;
-                while (x1 < ie && (acc < chunk || x1 == x0)) acc += item_cost(i2[x1++], hb);
-                if (x1 < n1) breaks.push_back(x1);
-                x0 = x1;
-              }
-            size_t nbk = t.bbeg;
-            for (int x = ib, gn = 0, gk = 0; x < n1; ++x) {
-              const bool brk = nbk < breaks.size() && breaks[nbk] == x;
-              if (brk) ++nbk;
-              if (gn == 0 || brk || gn >= group_items || gk + i2[x].kp > kGroupK) {
-                starts.push_back(x);
-                gn = gk = 0;
-              }
-              ++gn;
-              gk += i2[x].kp;
-            }
-          }
-          t.bend = (int)breaks.size();
-          std::vector<int> at;  // this tile's cuts: the sector's, moved back to a group start
-          for (int x : cuts) {
-            if (x > ib && x < n1 && !plan.tcx) x = *(std::upper_bound(starts.begin(), starts.end(), x) - 1);
-            at.push_back(x);
-          }
+          mma += 3.0 * 2.0 * 128 * tc_round16(hb) * pk.back();
+          const Groups& G = groups_of(hb);
+          const std::vector<int>& at = G.at;
+          const double ck = per_k(ha, hb);
+          t.bbeg = G.bbeg;
+          t.bend = G.bend;
           int np = 0;
           for (size_t c = 0; c + 1 < at.size(); ++c) np += at[c + 1] > at[c] ? 1 : 0;
           TcTile tl{};
@@ -1920,8 +1843,8 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
             TcTask u = t;
             u.ibeg = at[c];
             u.iend = at[c + 1];
-            double cost = 0.0;
-            for (int x = u.ibeg; x < u.iend; ++x) cost += stream_cost(i2[x], ha, hb);
+            const int x0 = u.ibeg - ib, x1 = u.iend - ib;
+            const double cost = pt[x1] - pt[x0] + ck * (pk[x1] - pk[x0]);
             if (np <= 1) {
               u.direct = 1;
               u.out_off = S.offset;
@@ -1973,21 +1896,7 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
     } else {
       schedule_lpt(c1, H.bundle1, bps * nsm, o1, r1);
     }
-    if (pairs) {
-      // pairs to clusters of two blocks; block 2c runs the first task of
-      // each of cluster c's pairs, block 2c + 1 the second
-      std::vector<int> op;
-      std::vector<int2> rp;
-      schedule_lpt(cp, bundle_p, bps * nsm / 2, op, rp);
-      o2.clear();
-      r2.clear();
-      for (const int2& g : rp)
-        for (int rank = 0; rank < 2; ++rank) {
-          const int b0 = (int)o2.size();
-          for (int k = g.x; k < g.y; ++k) o2.push_back(2 * op[k] + rank);
-          r2.push_back(make_int2(b0, (int)o2.size()));
-        }
-    } else if (kn.waves) {
+    if (kn.waves) {
       schedule_waves(c2, bps * nsm, o2, r2);
     } else {
       schedule_list(c2, bps * nsm, o2, r2);
@@ -2055,8 +1964,7 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
           base.out_base = T.out_off;
           base.out_ld = base.h_b;
         }
-        const uint8_t f0 = (uint8_t)((T.direct ? kTcDirect : 0) | (phase == 1 && T.stacked ? kTcStacked : 0) |
-                                     (phase == 2 && T.ghost ? kTcGhost : 0));
+        const uint8_t f0 = (uint8_t)((T.direct ? kTcDirect : 0) | (phase == 1 && T.stacked ? kTcStacked : 0));
         if (T.ibeg == T.iend) {
           TcWork x = base;
           x.flags = (uint8_t)(f0 | kTcFirst | kTcLast | kTcEmpty);
@@ -2069,8 +1977,8 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
           while (nbk < T.bend && breaks[nbk] <= i) ++nbk;
           const TcItem& it = items[i];
           TcWork x = base;
-          x.a_base = it.a_off + 2 * (int64_t)kTcRowsA * T.tm * it.kp;
-          x.b_base = it.b_off + 2 * (int64_t)nb * T.tn * it.kp;
+          x.a_base = (int64_t)(plan.tc_pool[it.a_pool] + it.a_off + 2 * (int64_t)kTcRowsA * T.tm * it.kp);
+          x.b_base = (int64_t)(plan.tc_pool[it.b_pool] + it.b_off + 2 * (int64_t)nb * T.tn * it.kp);
           x.kp = it.kp;
           x.alpha = it.alpha;
           x.a_pool = it.a_pool;
@@ -2170,22 +2078,6 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
   } else {
     flatten(1, t1, i1, o1, r1, w1, wr1);
     flatten(2, t2, i2, o2, r2, w2, wr2);
-    if (pairs) {
-      // the two blocks of a cluster must stream the same A pieces in the
-      // same order (their stages are filled for each other)
-      if (wr2.size() % 2) throw std::runtime_error("tensor-core plan: odd number of blocks for cluster pairs");
-      for (size_t c = 0; c + 1 < wr2.size(); c += 2) {
-        const int2 a = wr2[c], bq = wr2[c + 1];
-        if (a.y - a.x != bq.y - bq.x) throw std::runtime_error("tensor-core plan: cluster pair streams differ");
-        for (int i = 0; i < a.y - a.x; ++i) {
-          const TcWork& x = w2[a.x + i];
-          const TcWork& y = w2[bq.x + i];
-          const int fx = x.flags & ~(kTcGhost | kTcDirect), fy = y.flags & ~(kTcGhost | kTcDirect);
-          if (x.a_base != y.a_base || x.kp != y.kp || x.h_a != y.h_a || x.a_pool != y.a_pool || fx != fy)
-            throw std::runtime_error("tensor-core plan: cluster pair streams differ");
-        }
-      }
-    }
   }
   for (auto* d : {&plan.tc_w1, &plan.tc_w2}) d->release(stream_);
   for (auto* d : {&plan.tc_r1, &plan.tc_r2}) d->release(stream_);
@@ -2215,7 +2107,6 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
   plan.tc_l2 = std::move(l2);
   plan.tc_knobs = kn;
   plan.tc_knobs.nb = nb;
-  plan.tc_pairs = pairs;
   {
     int64_t full = 0;
     for (const TcItem& it : i2) full += it.a_pool == kTcPoolS ? 1 : 0;
@@ -2404,11 +2295,7 @@ void GpuEngine::sigma_tc(const Superblock& sb, SigmaPlan& p, const double* psi, 
   } else {
     cuda_check(dev::launch_tc_sigma(1, p.tc_nb, b, p.tc_w1.d, p.tc_r1.d, (int)p.tc_r1.n, out, kWaitLimitNs, stream_, p.tc_most[0]),
                "tc phase 1");
-    if (p.tc_pairs)
-      cuda_check(dev::launch_tc_sigma_pairs(b, p.tc_w2.d, p.tc_r2.d, (int)p.tc_r2.n, out, kWaitLimitNs, stream_, p.tc_most[1]),
-                 "tc phase 2 (cluster pairs)");
-    else
-      cuda_check(dev::launch_tc_sigma(2, p.tc_nb, b, p.tc_w2.d, p.tc_r2.d, (int)p.tc_r2.n, out, kWaitLimitNs, stream_, p.tc_most[1]),
+    cuda_check(dev::launch_tc_sigma(2, p.tc_nb, b, p.tc_w2.d, p.tc_r2.d, (int)p.tc_r2.n, out, kWaitLimitNs, stream_, p.tc_most[1]),
                  "tc phase 2");
   }
   if (marks) cuda_check(cudaEventRecord(marks[1], stream_), "record");

@@ -1,6 +1,7 @@
 // tcgen05 building blocks: a single-tile GEMM used to check the operand
 // layout, descriptors and TMEM read-back against a host product.
 #include <algorithm>
+#include <type_traits>
 
 #include "k_tc.cuh"
 #include "tc.cuh"
@@ -235,11 +236,11 @@ struct TcCfg {
   static constexpr uint32_t kTmemCols = kAcc * NB;
   static constexpr int kBlocksPerSm = NB == 64 ? 2 : 1;
 };
-constexpr int kTcMaxSlots = 16;
+constexpr int kTcSlots = 16;  // stages at most
 constexpr int kTcMaxAcc = 4;
 
 struct TcShared {
-  uint64_t full[kTcMaxSlots], empty[kTcMaxSlots], acc_full[kTcMaxAcc], acc_empty[kTcMaxAcc], drain;
+  uint64_t full[kTcSlots], empty[kTcSlots], acc_full[kTcMaxAcc], acc_empty[kTcMaxAcc], drain;
   uint32_t tbase;
   int abort_flag;
 };
@@ -347,7 +348,7 @@ __device__ __forceinline__ EpiRec load_epi(const TcWork* __restrict__ w, int i, 
 // 3500 clocks a 128 x 128 item (24 orbitals, M=500: 331 items an SM, 680 us).
 // The pairs now stay in registers, 64 columns a thread, folded two values an
 // instruction.
-template <int PHASE, int NB, bool PAIR = false>
+template <int PHASE, int NB>
 __global__ void __launch_bounds__(TcCfg<NB>::kThreads, TcCfg<NB>::kBlocksPerSm)
     tc_sigma_kernel(TcBufs b, const TcWork* __restrict__ work, const int2* __restrict__ ranges,
                     double* __restrict__ sigma, uint64_t limit_ns, int slots, uint32_t stage_bytes, int piece_k) {
@@ -364,7 +365,7 @@ __global__ void __launch_bounds__(TcCfg<NB>::kThreads, TcCfg<NB>::kBlocksPerSm)
   if (tid == 0) {
     for (int i = 0; i < slots; ++i) {
       mbar_init(&sh.full[i], 1);
-      mbar_init(&sh.empty[i], PAIR ? 2 : 1);  // pairs: released by both blocks' MMAs
+      mbar_init(&sh.empty[i], 1);
     }
     for (int i = 0; i < kTcAcc; ++i) {
       mbar_init(&sh.acc_full[i], 1);
@@ -377,9 +378,6 @@ __global__ void __launch_bounds__(TcCfg<NB>::kThreads, TcCfg<NB>::kBlocksPerSm)
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
-  // pairs: both blocks' barriers exist before either block copies or commits into the other
-  if (PAIR) cluster_sync();
-  const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
   const uint32_t tmem = sh.tbase;
   volatile int* abort_flag = &sh.abort_flag;
 
@@ -397,35 +395,19 @@ __global__ void __launch_bounds__(TcCfg<NB>::kThreads, TcCfg<NB>::kBlocksPerSm)
         n0 = n1;
         n1 = load_copy(work, i + 2, rg.y);
         if ((r.pf >> 16) & kTcEmpty) continue;
-        const int h_a = r.hw & 0xffff, h_b = (r.hw >> 16) & 0xffff, kp = r.kp;
-        const uint8_t* pa =
-            reinterpret_cast<const uint8_t*>(pick(b.pool, r.pf & 0xff) + join64(r.base.x, r.base.y));
-        const uint8_t* pb =
-            reinterpret_cast<const uint8_t*>(pick(b.pool, (r.pf >> 8) & 0xff) + join64(r.base.z, r.base.w));
-        for (int k0 = 0; k0 < kp; k0 += piece_k, ++k) {
-          const int w = min(piece_k, kp - k0);  // its K-chunks lie one after another
-          const uint32_t abytes = 4u * h_a * w, bbytes = 4u * h_b * w;
+        const uint32_t a4 = 4u * (r.hw & 0xffff), b4 = 4u * ((r.hw >> 16) & 0xffff);  // bytes per column
+        const uint8_t* pa = reinterpret_cast<const uint8_t*>(join64(r.base.x, r.base.y));
+        const uint8_t* pb = reinterpret_cast<const uint8_t*>(join64(r.base.z, r.base.w));
+        for (int left = r.kp; left > 0; left -= piece_k, ++k) {
+          const uint32_t w = (uint32_t)min(piece_k, left);  // its K-chunks lie one after another
+          const uint32_t abytes = a4 * w, bbytes = b4 * w;
           if (!tc_wait(&sh.empty[slot], ph ^ 1u, abort_flag, b.status, limit_ns)) {
             ok = false;
             break;
           }
           uint8_t* dst = smem + (uint32_t)slot * stage_bytes;
           mbar_expect_tx(&sh.full[slot], abytes + bbytes);
-          if constexpr (PAIR) {
-            // this block's half of the A piece's 8-column groups (hi and
-            // lo slices), into the same stage of both blocks of the pair
-            // (piece_k is one chunk)
-            const int ng = w / 8;
-            const int g0 = rank ? (ng + 1) / 2 : 0, g1 = rank ? ng : (ng + 1) / 2;
-            if (g1 > g0) {
-              const uint32_t slice = (uint32_t)h_a * w * 2;
-              const uint32_t off = (uint32_t)g0 * h_a * 16, len = (uint32_t)(g1 - g0) * h_a * 16;
-              bulk_g2s_mc(dst + off, pa + off, len, &sh.full[slot], (uint16_t)3);
-              bulk_g2s_mc(dst + slice + off, pa + slice + off, len, &sh.full[slot], (uint16_t)3);
-            }
-          } else {
-            bulk_g2s(dst, pa, abytes, &sh.full[slot]);
-          }
+          bulk_g2s(dst, pa, abytes, &sh.full[slot]);
           bulk_g2s(dst + abytes, pb, bbytes, &sh.full[slot]);
           pa += abytes;
           pb += bbytes;
@@ -440,19 +422,15 @@ __global__ void __launch_bounds__(TcCfg<NB>::kThreads, TcCfg<NB>::kBlocksPerSm)
         // copies already issued still land in shared memory: wait for them
         for (uint32_t i = (k > ns ? k - ns : 0); i < k; ++i)
           mbar_wait_bounded(&sh.full[i % ns], (i / ns) & 1u, limit_ns);
-      } else if (PAIR) {
-        // the last stages released by both blocks: every multicast copy of
-        // this block has landed in the partner and been read there
-        for (uint32_t i = (k > ns ? k - ns : 0); i < k; ++i)
-          tc_wait(&sh.empty[i % ns], (i / ns) & 1u, abort_flag, b.status, limit_ns);
       }
     }
   } else if (warp == kTcIssuer) {
-    // ---- MMA issuer: the whole warp walks the records and one lane issues.
-    // An MMA takes its descriptors from uniform registers: in code that one
-    // lane runs by itself every operand is moved there before every MMA,
-    // about 70 clocks an MMA whatever its width, which bounded both phases
-    // (24 orbitals, M=500: 490 clocks for the six MMAs of a piece).
+    // ---- MMA issuer: the whole warp walks the records and one lane issues
+    // (mma_bf16_if).  The issue of an MMA blocks while the one before it runs
+    // (64 clocks at 128 x 128, 48 at 128 x 64), so that every clock spent
+    // between two pieces is lost to the tensor core: the next piece's record,
+    // place and descriptors are worked out between the MMAs of this one.
+    const bool on = elect_one();
     int slot = 0;
     uint32_t ph = 0;
     int ab = 0;
@@ -462,91 +440,87 @@ __global__ void __launch_bounds__(TcCfg<NB>::kThreads, TcCfg<NB>::kBlocksPerSm)
     // low words of the operands' descriptors: address / 16 and rows (the
     // leading byte offset / 16); the high word is the same for all
     constexpr uint64_t kDescHi = smem_desc_hi();
-    // One piece per step.  The next piece's record and the state of its barrier
-    // are looked at behind the first three MMAs of this one: the queue of the
-    // tensor core is short, and what is done with it empty costs twice.
+    // records i (uniform in u_*), i + 1 (n0) and i + 2 (n1) are on their way
     MmaRec n0 = load_mma(work, rg.x, rg.y), n1 = load_mma(work, rg.x + 1, rg.y);
-    int i = rg.x, kp = 0, k0 = 0, flags = 0;
-    uint32_t h_a = 0, h_b = 0, idesc = 0;
-    bool ready = false;
+    int u_kp = uniform(n0.kp), u_hw = uniform(n0.hw), u_pf = uniform(n0.pf);
+    n0 = n1;
+    n1 = load_mma(work, rg.x + 2, rg.y);
+    int i = rg.x, kp = 0, k0 = 0, flags = 0, w = 0;
+    uint32_t ha = 0, hb = 0, idesc = 0, la = 0, lb = 0;
     auto next_item = [&]() {  // false at the end of the records
       do {
         if (i >= rg.y) return false;
-        const int pf = uniform(n0.pf), hw = uniform(n0.hw);
-        kp = uniform(n0.kp);
+        kp = u_kp;
+        ha = (uint32_t)u_hw & 0xffffu;
+        hb = (uint32_t)u_hw >> 16;
+        flags = (u_pf >> 16) & 0xff;
+        ++i;
+        u_kp = uniform(n0.kp);
+        u_hw = uniform(n0.hw);
+        u_pf = uniform(n0.pf);
         n0 = n1;
         n1 = load_mma(work, i + 2, rg.y);
-        ++i;
-        flags = (pf >> 16) & 0xff;
-        h_a = (uint32_t)hw & 0xffffu;
-        h_b = (uint32_t)hw >> 16;
       } while (flags & kTcEmpty);
-      idesc = idesc0 | ((((h_b + 15u) & ~15u) >> 3) << 17);
+      idesc = idesc0 | ((((hb + 15u) & ~15u) >> 3) << 17);
       k0 = 0;
       return true;
     };
-    bool more = next_item();
+    auto place = [&]() {  // the piece at k0, in stage `slot`
+      w = min(piece_k, kp - k0);
+      const uint32_t a0 = sm0 + (uint32_t)slot * stage16;
+      la = a0 | (ha << 16);
+      lb = (a0 + (ha * (uint32_t)w >> 2)) | (hb << 16);
+    };
+    bool more = next_item(), ready = false;
+    if (more) place();
     while (more) {
-      if (k0 == 0 && (flags & kTcGStart) &&
-          !__all_sync(0xffffffffu, tc_wait(&sh.acc_empty[ab], aph ^ 1u, abort_flag, b.status, limit_ns)))
+      const bool gstart = k0 == 0 && (flags & kTcGStart);
+      if (gstart && !__all_sync(0xffffffffu, tc_wait(&sh.acc_empty[ab], aph ^ 1u, abort_flag, b.status, limit_ns)))
         break;
       if (!ready && !__all_sync(0xffffffffu, tc_wait(&sh.full[slot], ph, abort_flag, b.status, limit_ns))) break;
       fence_after_sync();
-      const uint32_t a0 = sm0 + (uint32_t)slot * stage16;
-      const int w = min(piece_k, kp - k0);
-      const uint32_t b0 = a0 + (h_a * (uint32_t)w >> 2);  // 16-byte units
-      const uint32_t d = tmem + (uint32_t)ab * (uint32_t)NB;
-      const uint32_t idesc_c = idesc, ha = h_a, hb = h_b;
+      const uint32_t d = tmem + (uint32_t)ab * (uint32_t)NB, id = idesc;
+      const int w0 = min(kTcKC, w), w1 = w - w0;
+      // a slice of h rows x w0 columns is h w0 / 8 units; one K=16 step 2 h
+      const uint64_t dah = kDescHi | la, dal = dah + (ha * (uint32_t)w0 >> 3);
+      const uint64_t dbh = kDescHi | lb, dbl = dbh + (hb * (uint32_t)w0 >> 3);
+      const uint64_t sa = 2 * ha, sb = 2 * hb;
+      const uint64_t ea = dah + 4 * sa, eb = dbh + 4 * sb;  // second chunk
+      const uint64_t eal = ea + (ha * (uint32_t)w1 >> 3), ebl = eb + (hb * (uint32_t)w1 >> 3);
       const bool gend = (flags & kTcGEnd) && k0 + w >= kp;
-      const uint32_t acc0 = (k0 == 0 && (flags & kTcGStart)) ? 0u : 1u;
       const int slot_c = slot, ab_c = ab;
-      const uint32_t la = a0 | (ha << 16), lb = b0 | (hb << 16);
-      const int w0 = min(kTcKC, w);
-      // a slice of h rows x w0 columns is h w0 / 8 units
-      const uint64_t dah = kDescHi | la, dal = kDescHi | (la + (ha * (uint32_t)w0 >> 3));
-      const uint64_t dbh = kDescHi | lb, dbl = kDescHi | (lb + (hb * (uint32_t)w0 >> 3));
-      if (elect_one()) {
-        mma_bf16(d, dah, dbh, idesc_c, acc0);
-        mma_bf16(d, dah, dbl, idesc_c, 1u);
-        mma_bf16(d, dal, dbh, idesc_c, 1u);
-      }
-      __syncwarp();
-      if (++slot == slots) {
-        slot = 0;
-        ph ^= 1u;
-      }
-      const bool probe = mbar_test(&sh.full[slot], ph);
+      mma_bf16_if(on, d, dah, dbh, id, gstart ? 0u : 1u);
+      k0 += w;
       if (gend && ++ab == kTcAcc) {
         ab = 0;
         aph ^= 1u;
       }
-      k0 += w;
-      if (k0 >= kp) more = next_item();
-      if (elect_one()) {
-        const uint64_t sa = 2 * ha, sb = 2 * hb;  // one K=16 step
-        if (w0 == kTcKC) {
-          mma_bf16(d, dah + sa, dbh + sb, idesc_c, 1u);
-          mma_bf16(d, dah + sa, dbl + sb, idesc_c, 1u);
-          mma_bf16(d, dal + sa, dbh + sb, idesc_c, 1u);
-        }
-        if (w > kTcKC) {  // the second chunk
-          const uint32_t w1 = (uint32_t)w - kTcKC;
-          const uint64_t eah = dah + 8 * ha, eal = eah + (ha * w1 >> 3);
-          const uint64_t ebh = dbh + 8 * hb, ebl = ebh + (hb * w1 >> 3);
-          mma_bf16(d, eah, ebh, idesc_c, 1u);
-          mma_bf16(d, eah, ebl, idesc_c, 1u);
-          mma_bf16(d, eal, ebh, idesc_c, 1u);
-          if (w1 == kTcKC) {
-            mma_bf16(d, eah + sa, ebh + sb, idesc_c, 1u);
-            mma_bf16(d, eah + sa, ebl + sb, idesc_c, 1u);
-            mma_bf16(d, eal + sa, ebh + sb, idesc_c, 1u);
-          }
-        }
-        if (PAIR) mma_commit_mc(&sh.empty[slot_c], (uint16_t)3);
-        else mma_commit(&sh.empty[slot_c]);
-        if (gend) mma_commit(&sh.acc_full[ab_c]);
+      if (++slot == slots) {
+        slot = 0;
+        ph ^= 1u;
       }
-      __syncwarp();
+      mma_bf16_if(on, d, dah, dbl, id, 1u);
+      if (k0 >= kp) more = next_item();
+      mma_bf16_if(on, d, dal, dbh, id, 1u);
+      if (more) place();
+      if (w0 == kTcKC) {
+        mma_bf16_if(on, d, dah + sa, dbh + sb, id, 1u);
+        mma_bf16_if(on, d, dah + sa, dbl + sb, id, 1u);
+        mma_bf16_if(on, d, dal + sa, dbh + sb, id, 1u);
+      }
+      if (w1 > 0) {
+        mma_bf16_if(on, d, ea, eb, id, 1u);
+        mma_bf16_if(on, d, ea, ebl, id, 1u);
+        mma_bf16_if(on, d, eal, eb, id, 1u);
+        if (w1 == kTcKC) {
+          mma_bf16_if(on, d, ea + sa, eb + sb, id, 1u);
+          mma_bf16_if(on, d, ea + sa, ebl + sb, id, 1u);
+          mma_bf16_if(on, d, eal + sa, eb + sb, id, 1u);
+        }
+      }
+      const bool probe = mbar_test(&sh.full[slot], ph);
+      mma_commit_if(on, &sh.empty[slot_c]);
+      if (gend) mma_commit_if(on, &sh.acc_full[ab_c]);
       ready = __all_sync(0xffffffffu, probe);
     }
   } else {
@@ -560,10 +534,24 @@ __global__ void __launch_bounds__(TcCfg<NB>::kThreads, TcCfg<NB>::kBlocksPerSm)
     uint32_t aph = 0;
     bool ok = true, first = true;
     uint64_t vh[PHASE == 2 ? 32 : 1], vl[PHASE == 2 ? 32 : 1];
-    EpiRec nx = load_epi(work, rg.x, rg.y);
+    // the row map of a stacked phase-1 tile is read one record ahead as well
+    auto load_row = [&](const EpiRec& x) {
+      const bool st = PHASE == 1 && ((x.pf >> 16) & kTcStacked) && row < (x.q2.x & 0xffff);
+      return st ? __ldg(reinterpret_cast<const int4*>(b.rows + join64(x.q1.x, x.q1.y) + row)) : make_int4(0, 0, 0, 0);
+    };
+    EpiRec n0 = load_epi(work, rg.x, rg.y), n1{};
+    int4 row_next = load_row(n0);
+    if (PHASE == 1) n1 = load_epi(work, rg.x + 1, rg.y);
     for (int i = rg.x; i < rg.y && ok; ++i) {
-      const EpiRec r = nx;
-      nx = load_epi(work, i + 1, rg.y);
+      const EpiRec r = n0;
+      const int4 row_map = row_next;
+      if (PHASE == 1) {
+        n0 = n1;
+        n1 = load_epi(work, i + 2, rg.y);
+        row_next = load_row(n0);
+      } else {
+        n0 = load_epi(work, i + 1, rg.y);
+      }
       const int flags = (r.pf >> 16) & 0xff;
       if (!(flags & (kTcFirst | kTcLast | kTcGEnd))) continue;
       const float alpha = __int_as_float(r.q1.w);
@@ -611,7 +599,7 @@ __global__ void __launch_bounds__(TcCfg<NB>::kThreads, TcCfg<NB>::kBlocksPerSm)
 #pragma unroll
           for (int e = 0; e < 32; ++e) vh[e] = vl[e] = 0ull;
         }
-        if (last && !(PAIR && (flags & kTcGhost))) {
+        if (last) {
           const int64_t out_base = join64(r.q1.x, r.q1.y);
           const int vrc = r.q2.y, out_ld = r.q2.z;
           const bool direct = (flags & kTcDirect) != 0;
@@ -648,48 +636,53 @@ __global__ void __launch_bounds__(TcCfg<NB>::kThreads, TcCfg<NB>::kBlocksPerSm)
         int s_h = h_a, s_row = row;
         float s_alpha = alpha;
         if ((flags & kTcStacked) && row < h_a) {
-          const int4 e = __ldg(reinterpret_cast<const int4*>(b.rows + out_base + row));
-          s_base = (int64_t)(((uint64_t)(uint32_t)e.y << 32) | (uint32_t)e.x);
-          s_h = e.z & 0xffff;
-          s_row = (e.z >> 16) & 0xffff;
-          s_alpha = __int_as_float(e.w);
+          s_base = join64(row_map.x, row_map.y);
+          s_h = row_map.z & 0xffff;
+          s_row = (row_map.z >> 16) & 0xffff;
+          s_alpha = __int_as_float(row_map.w);
         }
         const bool mine = row < h_a && s_h > 0;
-        const int ncols = min(NB, out_ld - col0) - cw;  // S columns of this warp (a multiple of 8)
-        __nv_bfloat16* sp = b.pool[kTcPoolS] + s_base;
+        const int c_s = col0 + cw;                      // S column of this warp's first
+        const int ncols = min(NB, out_ld - col0) - cw;  // its S columns (a multiple of 8)
+        // element of the row in the first 8-column group of its K-chunk; the
+        // next group is 8 s_h on, the lo slice s_h wc, the next chunk 64 s_h
+        __nv_bfloat16* sp = b.pool[kTcPoolS] + s_base + 2 * (int64_t)s_h * c_s + (s_row >> 3) * 64 + (s_row & 7) * 8;
+        auto store = [&](auto fp16) {
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          float v[16];
-          if (g < ng) {
-            tmem_ld16(d + 16u * (uint32_t)g, v);
-            if (g == ng - 1) {
-              fence_before_sync();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&sh.acc_empty[ab]);
-            }
-          }
-#pragma unroll
-          for (int g8 = 0; g8 < 2; ++g8) {
-            const int c0 = 16 * g + 8 * g8;  // column in this warp's 64
-            if (mine && c0 < ncols) {
-              // columns of the accumulator beyond h_b (a multiple of 8) are
-              // another operand's: zeros
-              const bool zero = cw + c0 >= h_b;
-              uint32_t hw4[4], lw4[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const uint64_t x =
-                    zero ? 0ull : scale2(s_alpha, v[8 * g8 + 2 * e], v[8 * g8 + 2 * e + 1]);
-                split16x2(x, b.fp16 != 0, hw4[e], lw4[e]);
+          for (int g = 0; g < 4; ++g) {
+            float v[16];
+            if (g < ng) {
+              tmem_ld16(d + 16u * (uint32_t)g, v);
+              if (g == ng - 1) {
+                fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sh.acc_empty[ab]);
               }
-              const int Cc = col0 + cw + c0;  // S column
-              const int cc = Cc / kTcKC, wc = min(kTcKC, out_ld - kTcKC * cc);
-              const int64_t off = 2 * (int64_t)s_h * kTcKC * cc + (kmajor_off(s_row, Cc % kTcKC, s_h) >> 1);
-              *(uint4*)(sp + off) = make_uint4(hw4[0], hw4[1], hw4[2], hw4[3]);
-              *(uint4*)(sp + off + (int64_t)s_h * wc) = make_uint4(lw4[0], lw4[1], lw4[2], lw4[3]);
+            }
+            const int cc = 32 * (g / 2);
+            const int wc = min(kTcKC, out_ld - c_s - cc);
+#pragma unroll
+            for (int g8 = 0; g8 < 2; ++g8) {
+              const int c0 = 16 * g + 8 * g8;  // column in this warp's 64
+              if (mine && c0 < ncols) {
+                // columns of the accumulator beyond h_b (a multiple of 8) are
+                // another operand's: zeros
+                const bool zero = cw + c0 >= h_b;
+                uint32_t hw4[4], lw4[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const uint64_t x = zero ? 0ull : scale2(s_alpha, v[8 * g8 + 2 * e], v[8 * g8 + 2 * e + 1]);
+                  split16x2(x, decltype(fp16)::value, hw4[e], lw4[e]);
+                }
+                __nv_bfloat16* q = sp + 2 * cc * s_h + (c0 - cc) * s_h;
+                *(uint4*)q = make_uint4(hw4[0], hw4[1], hw4[2], hw4[3]);
+                *(uint4*)(q + wc * s_h) = make_uint4(lw4[0], lw4[1], lw4[2], lw4[3]);
+              }
             }
           }
-        }
+        };
+        if (b.fp16) store(std::true_type{});
+        else store(std::false_type{});
         if (ng == 0 && lane == 0) mbar_arrive(&sh.acc_empty[ab]);
       }
       if (have && ++ab == kTcAcc) {
@@ -710,23 +703,20 @@ __global__ void __launch_bounds__(TcCfg<NB>::kThreads, TcCfg<NB>::kBlocksPerSm)
     fence_after_sync();
     tmem_dealloc(tmem, TcCfg<NB>::kTmemCols);
   }
-  // pairs: neither block leaves while the other may still copy into it
-  if (PAIR) cluster_sync();
 }
 
 // Columns per piece and stages of the ring for pieces of at most rows rows (A
 // and B together) and kp columns: two K-chunks a piece, which halves the
-// barrier round trips, where three stages of them fit (always with 128-column
-// tiles; with 64 for the pieces of small sectors), else one.
+// barrier round trips, where three stages of them fit, else one.
 struct TcRing {
   int piece_k, stage, slots;
 };
 template <int NB>
-static TcRing tc_ring(int rows, int kp, bool pair) {
+static TcRing tc_ring(int rows, int kp) {
   TcRing r;
-  for (r.piece_k = pair ? kTcKC : 2 * kTcKC;; r.piece_k = kTcKC) {
+  for (r.piece_k = 2 * kTcKC;; r.piece_k = kTcKC) {
     r.stage = (4 * rows * std::min(r.piece_k, kp) + 127) / 128 * 128;
-    r.slots = std::min(kTcMaxSlots, TcCfg<NB>::kRing / r.stage);
+    r.slots = std::min(kTcSlots, TcCfg<NB>::kRing / r.stage);
     if (r.slots >= 3 || r.piece_k == kTcKC) return r;
   }
 }
@@ -736,11 +726,11 @@ static cudaError_t launch_tc_sigma_nb(const TcBufs& b, const TcWork* work, const
                                       double* sigma, uint64_t limit_ns, cudaStream_t s, int2 most) {
   constexpr int smem = TcCfg<NB>::kSmem;
   if (most.x <= 0 || most.x > kTcRowsA + NB || most.y <= 0) return cudaErrorInvalidValue;
-  const TcRing r = tc_ring<NB>(most.x, most.y, false);
+  const TcRing r = tc_ring<NB>(most.x, most.y);
   cudaError_t e = cudaFuncSetAttribute(tc_sigma_kernel<PHASE, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  tc_sigma_kernel<PHASE, NB><<<nblocks, TcCfg<NB>::kThreads, smem, s>>>(b, work, ranges, sigma, limit_ns, r.slots,
-                                                                       (uint32_t)r.stage, r.piece_k);
+  tc_sigma_kernel<PHASE, NB>
+      <<<nblocks, TcCfg<NB>::kThreads, smem, s>>>(b, work, ranges, sigma, limit_ns, r.slots, (uint32_t)r.stage, r.piece_k);
   return cudaGetLastError();
 }
 
@@ -755,33 +745,6 @@ cudaError_t launch_tc_sigma(int phase, int nb, const TcBufs& b, const TcWork* wo
 }
 
 int tc_blocks_per_sm(int nb) { return nb == 64 ? TcCfg<64>::kBlocksPerSm : TcCfg<128>::kBlocksPerSm; }
-
-cudaError_t launch_tc_sigma_pairs(const TcBufs& b, const TcWork* work, const int2* ranges, int nblocks, double* sigma,
-                                  uint64_t limit_ns, cudaStream_t s, int2 most) {
-  if (nblocks <= 0) return cudaGetLastError();
-  if (most.x <= 0 || most.x > 2 * kTcRowsA || most.y <= 0) return cudaErrorInvalidValue;
-  const TcRing r = tc_ring<128>(most.x, most.y, true);
-  if (nblocks % 2) return cudaErrorInvalidValue;
-  constexpr int smem = TcCfg<128>::kSmem;
-  auto kern = tc_sigma_kernel<2, 128, true>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nblocks);
-  cfg.blockDim = dim3(TcCfg<128>::kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, kern, b, work, ranges, sigma, limit_ns, r.slots, (uint32_t)r.stage, r.piece_k);
-  if (e != cudaSuccess) return e;
-  return cudaGetLastError();
-}
 
 // Bound by the latency of the slot reads: few tiles (56 at 24 orbitals,
 // M=500) with tens of partials each, so every thread keeps eight reads in

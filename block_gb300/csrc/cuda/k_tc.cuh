@@ -90,7 +90,6 @@ struct TcTask {
   int32_t out_kp, direct;
   int32_t valid_rows, valid_cols;
   int32_t stacked;
-  int32_t ghost;  // cluster pairs: repeats its partner's tile, writes nothing
   int32_t bbeg, bend;  // phase 2: the tile's group breaks in the host plan's list
 };
 
@@ -115,7 +114,8 @@ struct TcTile {
 // block's tasks, flattened in processing order, each carrying what the
 // producer, MMA and epilogue roles need, so that a warp loads 32 of them
 // with one coalesced access and no role chases task -> item pointers.
-//   a_base / b_base: pool elements of the row tile (128 rows of A, 64 of B)
+//   a_base / b_base: device addresses of the row tile (128 rows of A, NB of B)
+//     in their pools
 //   out_base: phase 1: S row-tile base (pool S); phase 2 direct: sigma
 //     element of tile (0, 0); phase 2 partial: partial slot (float2)
 //   out_ld: phase 1: kp of S; phase 2 direct: sigma row stride; partial: h_b
@@ -130,8 +130,7 @@ enum : uint32_t {
   kTcEmpty = 8,    // task without items (writes zeros)
   kTcGStart = 16,  // first item of an accumulation group
   kTcGEnd = 32,    // last item of an accumulation group
-  kTcStacked = 64,  // phase 1: A is a stack of operators; out_base indexes TcBufs::rows
-  kTcGhost = 128    // cluster pairs: this block repeats its partner's tile and writes nothing
+  kTcStacked = 64   // phase 1: A is a stack of operators; out_base indexes TcBufs::rows
 };
 struct __align__(16) TcWork {
   int64_t a_base, b_base, out_base;
@@ -167,19 +166,11 @@ cudaError_t launch_tc_pack(const TcBufs& b, const TcPack* units, int nunits, cud
 // work[ranges[j].x .. ranges[j].y); nb = output-tile width (kTcRowsB or
 // kTcRowsBWide, the row tile of the B-role pools); limit_ns bounds every
 // pipeline wait; most: the most rows of A and B together and the most K of a
-// record (they size the ring's stages)
+// record (they set the pieces)
 cudaError_t launch_tc_sigma(int phase, int nb, const TcBufs& b, const TcWork* work, const int2* ranges, int nblocks,
                             double* sigma, uint64_t limit_ns, cudaStream_t s, int2 most);
 // persistent blocks per SM of the kernels with tile width nb
 int tc_blocks_per_sm(int nb);
-// Phase 2 with 128-column tiles on pairs of blocks in thread-block clusters
-// of two (blocks 2c and 2c + 1): the two blocks of a pair run record streams
-// of the same items (the column tiles tn and tn + 1, or a ghost copy, of one
-// sigma row tile); each copies half of every A piece into both blocks'
-// stages with a cluster-multicast bulk copy and its own B piece, and a stage
-// is refilled once both blocks' MMAs released it.  nblocks is even.
-cudaError_t launch_tc_sigma_pairs(const TcBufs& b, const TcWork* work, const int2* ranges, int nblocks, double* sigma,
-                                  uint64_t limit_ns, cudaStream_t s, int2 most);
 // Bounded-wait self-check: one thread waits, with the sigma kernels' wait,
 // on an mbarrier that nothing arrives at; out[0] = 1 when the wait gave up,
 // out[1] = nanoseconds waited; *status is set by the wait.
