@@ -410,6 +410,52 @@ struct PlanTimer {
 // operands) stay together on one block, consecutive, unless a bundle costs
 // more than a block's fair share, in which case it is cut into pieces of at
 // most that share.
+// Clocks of an exact item on its block: of each quarter of 32 TMEM lanes that
+// its rows take (read-out and sums), and of K times columns (MMAs).  Fitted to
+// the blocks' clocks at 20 orbitals M=300 (0.7 % rms in phase 1, 4 % in phase 2);
+// by K alone the slowest block of phase 2 took 1.23 times the mean.
+double tcx_quarter_clocks(int ha) { return 830.0 * ((ha + 31) / 32); }
+constexpr double kTcxKClocks = 1.44;
+
+// Order of one block's exact records.  A tile of ha rows keeps ceil(ha / 32) of
+// the four quarters of the epilogue warps busy with its sums, for longer than its
+// MMAs where K is short; the records of as many tasks as have quarters of their
+// own alternate, so that the sums of one run beside those of another (20 orbitals
+// M=300, with 8 epilogue warps and 64 columns: 1963 -> 1744 us a product).  rows and counts: of the tasks, in order;
+// emit(task, record of the task, first lane).
+template <class Emit>
+void interleave_tasks(const std::vector<int>& rows, const std::vector<int>& counts, Emit emit) {
+  struct Open {
+    int task, at, q, nq;
+  };
+  std::vector<Open> open;
+  unsigned used = 0;
+  size_t next = 0;
+  int q = 0;
+  while (next < rows.size() || !open.empty()) {
+    while (next < rows.size()) {
+      const int nq = (rows[next] + 31) / 32;
+      const unsigned mask = (1u << nq) - 1;
+      int s = -1;
+      for (int k = 0; k < 4 && s < 0; ++k) {
+        const int c = (q + k) & 3;
+        if (c + nq <= 4 && !(used & (mask << c))) s = c;
+      }
+      if (s < 0) break;
+      open.push_back({(int)next++, 0, s, nq});
+      used |= mask << s;
+      q = (s + nq) & 3;
+    }
+    size_t left = 0;
+    for (Open& o : open) {
+      emit(o.task, o.at, 32 * o.q);
+      if (++o.at == counts[o.task]) used &= ~(((1u << o.nq) - 1) << o.q);
+      else open[left++] = o;
+    }
+    open.resize(left);
+  }
+}
+
 void schedule_lpt(const std::vector<double>& cost, const std::vector<int64_t>& bundle, int nblocks,
                   std::vector<int>& order, std::vector<int2>& ranges) {
   const int n = (int)cost.size();
@@ -1238,6 +1284,9 @@ void GpuEngine::plan_tc(const Superblock& sb, SigmaPlan& plan) {
   });
   laps.lap("couplings");
   int64_t pool_n[kTcPools] = {0, 0, 0, 0, 0};
+  // rows of a B operand (columns of the tiles): the exact kernels' MMAs take
+  // several slices as columns, each a multiple of 16
+  auto round_cols = [&](int x) { return plan.tcx ? tc_round16(x) : tc_round8(x); };
   // Every item is checked against the packed operands it reads (rows and K
   // of its output sector), so that no bulk copy can leave its operand.
   auto fail = []() { throw std::runtime_error("tensor-core plan: operand shape does not match its sector"); };
@@ -1254,7 +1303,7 @@ void GpuEngine::plan_tc(const Superblock& sb, SigmaPlan& plan) {
     p.ld = v.ld;
     p.rows_v = v.rows;
     p.cols_v = v.cols;
-    p.rows_p = tc_round8(v.rows);
+    p.rows_p = pool == kTcPoolL ? tc_round8(v.rows) : round_cols(v.rows);
     p.kp = tc_round16(v.cols);
     p.trans = v.trans ? 1 : 0;
     p.rt = pool == kTcPoolL ? kTcRowsA : nb;  // L blocks are A operands, R blocks B operands
@@ -1292,7 +1341,7 @@ void GpuEngine::plan_tc(const Superblock& sb, SigmaPlan& plan) {
     t.trans = 1;
     t.rows_v = S.cols;
     t.cols_v = S.rows;
-    t.rows_p = tc_round8(S.cols);
+    t.rows_p = round_cols(S.cols);
     t.kp = tc_round16(S.rows);
     t.rt = nb;
     t.dst_off = psit_off[s] = pool_n[kTcPoolPsiT];
@@ -1315,7 +1364,7 @@ void GpuEngine::plan_tc(const Superblock& sb, SigmaPlan& plan) {
     for (const Coupling& c : cl) {
       if (c.va.identity && c.vb.identity) throw std::runtime_error("identity x identity pair term");
       const auto& SV = sb.sectors[c.vs];
-      const int out_rows_p = tc_round8(SV.rows), out_cols_p = tc_round8(SV.cols);
+      const int out_rows_p = tc_round8(SV.rows), out_cols_p = round_cols(SV.cols);
       TcItem it{};
       if (c.va.identity) {  // sigma(lQ,rQ) += f psi(lQ,rQ') B^T
         const TcPack pb = pack_view(1, c.vb, rmap);
@@ -1348,7 +1397,7 @@ void GpuEngine::plan_tc(const Superblock& sb, SigmaPlan& plan) {
         it.a_ex = pa.ex_off;
         it.b_ex = psit_ex[c.cs];
         const auto& C = sb.sectors[c.cs];
-        if (pa.rows_p != out_rows_p || pa.kp != it.kp || tc_round8(C.cols) != out_cols_p ||
+        if (pa.rows_p != out_rows_p || pa.kp != it.kp || round_cols(C.cols) != out_cols_p ||
             tc_round16(C.rows) != it.kp)
           fail();
         per_sector[c.vs].push_back(it);
@@ -1391,7 +1440,7 @@ void GpuEngine::plan_tc(const Superblock& sb, SigmaPlan& plan) {
         a.b_ex = psit_ex[c.cs];
         a.o_ex = cur_ex;
         const auto& C = sb.sectors[c.cs];
-        if (pa.rows_p != rows_p || pa.kp != a.kp || tc_round8(C.cols) != tc_round8(mc) ||
+        if (pa.rows_p != rows_p || pa.kp != a.kp || round_cols(C.cols) != round_cols(mc) ||
             tc_round16(C.rows) != a.kp)
           fail();
         const int idx = (int)i1.size();
@@ -1400,7 +1449,7 @@ void GpuEngine::plan_tc(const Superblock& sb, SigmaPlan& plan) {
           for (int tn = 0; tn < (mc + nb - 1) / nb; ++tn) {
             TcTask t{};
             t.a_rows = rows_p;
-            t.b_rows = tc_round8(mc);
+            t.b_rows = round_cols(mc);
             t.tm = tm;
             t.tn = tn;
             t.ibeg = idx;
@@ -1618,6 +1667,10 @@ void GpuEngine::plan_tc(const Superblock& sb, SigmaPlan& plan) {
     cuda_check(cudaMallocAsync((void**)&plan.tcx_t, (size_t)std::max<int64_t>(t_n, 1) * sizeof(double), stream_),
                "tcx stage-1 products");
     plan.tcx_tpack.upload(t_packs, stream_);
+    // most units have a few thousand elements: blocks by the mean unit, which
+    // gives a large one more passes (20 orbitals M=300, 25620 units, 4 blocks
+    // each: 249 us)
+    plan.tcx_t_split = t_packs.empty() ? 1 : (int)std::min<int64_t>(64, t_n / (2048 * (int64_t)t_packs.size()) + 1);
     TcxBufs xb{};
     xb.src[0] = arena(L);
     xb.src[1] = arena(R);
@@ -1689,6 +1742,7 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
   std::vector<int> sec2;
   std::vector<TcTile> tiles;
   std::vector<int64_t> slots;
+  auto round_cols = [&](int x) { return plan.tcx ? tc_round16(x) : tc_round8(x); };  // as packed (plan_tc)
   std::vector<int> breaks;  // per tile: items at which an accumulation group starts anew
   const int group_items = std::max(1, kn.group);
   constexpr int kGroupK = 1024;
@@ -1697,7 +1751,7 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
   for (int s = 0; s < nsec; ++s) {
     const auto& S = sb.sectors[s];
     for (int tn = 0; tn < (S.cols + nb - 1) / nb; ++tn) {
-      const int hb = std::min(nb, tc_round8(S.cols) - nb * tn);
+      const int hb = std::min(nb, round_cols(S.cols) - nb * tn);
       for (const TcItem& it : per_sector[s]) total += item_cost(it, hb) * ((S.rows + 127) / 128);
     }
   }
@@ -1711,9 +1765,14 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
     // alone the slowest block took 1.4 times the mean).
     // Sums over items of a sector come from prefix sums of what does not
     // depend on the tile (trips) and of K.
-    const double mma_step = (plan.tcx ? 21.0 : 3.0) / 16.0;
-    auto trips = [](const TcItem& it) { return 140.0 + 250.0 * ((it.kp + 63) / 64); };
-    auto per_k = [&](int ha, int hb) { return mma_step * (32.0 + tc_round16(hb) / 4.0) + 0.016 * (ha + hb); };
+    // The exact kernels' items cost their quarters of rows and their K times
+    // columns (tcx_quarter_clocks, tcx_k_clocks).
+    const double mma_step = 3.0 / 16.0;
+    auto trips = [&](const TcItem& it) { return plan.tcx ? 1.0 : 140.0 + 250.0 * ((it.kp + 63) / 64); };
+    auto trip = [&](int ha) { return plan.tcx ? tcx_quarter_clocks(ha) : 1.0; };
+    auto per_k = [&](int ha, int hb) {
+      return plan.tcx ? kTcxKClocks * hb : mma_step * (32.0 + tc_round16(hb) / 4.0) + 0.016 * (ha + hb);
+    };
     // Pieces: every tile of a sector is cut at about the same items, into
     // pieces of at most a kPieces-th of a block's share.  The pieces are laid
     // out piece by piece and, within one, tile by tile, and dealt to the blocks
@@ -1726,16 +1785,16 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
     double stream_total = 0.0;
     for (int s = 0; s < nsec; ++s) {
       const auto& S = sb.sectors[s];
-      const int rows_p = tc_round8(S.rows), cols_p = tc_round8(S.cols);
+      const int rows_p = tc_round8(S.rows), cols_p = round_cols(S.cols);
       double t = 0.0, k = 0.0;
       for (const TcItem& it : per_sector[s]) {
         t += trips(it);
         k += it.kp;
       }
-      sec_tile[s] = t + k * per_k(std::min(128, rows_p), std::min(nb, cols_p));
+      sec_tile[s] = t * trip(std::min(128, rows_p)) + k * per_k(std::min(128, rows_p), std::min(nb, cols_p));
       for (int tm = 0; tm < (S.rows + 127) / 128; ++tm)
         for (int tn = 0; tn < (S.cols + nb - 1) / nb; ++tn)
-          sec_cost[s] += t + k * per_k(std::min(128, rows_p - 128 * tm), std::min(nb, cols_p - nb * tn));
+          sec_cost[s] += t * trip(std::min(128, rows_p - 128 * tm)) + k * per_k(std::min(128, rows_p - 128 * tm), std::min(nb, cols_p - nb * tn));
       stream_total += sec_cost[s];
     }
     const int nblk = (plan.tcx ? tcx_blocks_per_sm() : tc_blocks_per_sm(nb)) * nsm;
@@ -1749,7 +1808,7 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
       const int ib = (int)i2.size();
       i2.insert(i2.end(), per_sector[s].begin(), per_sector[s].end());
       const int ie = (int)i2.size();
-      const int rows_p = tc_round8(S.rows), cols_p = tc_round8(S.cols);
+      const int rows_p = tc_round8(S.rows), cols_p = round_cols(S.cols);
       const int ntm = (S.rows + 127) / 128, ntn = (S.cols + nb - 1) / nb;
       std::vector<double> pt(ie - ib + 1, 0.0), pk(ie - ib + 1, 0.0);
       for (int x = ib; x < ie; ++x) {
@@ -1760,9 +1819,9 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
       std::vector<int> cuts{ib};
       if (sec_tile[s] > piece && ie - ib > 1) {
         const double per = sec_tile[s] / std::ceil(sec_tile[s] / piece);
-        const double ck = per_k(std::min(128, rows_p), std::min(nb, cols_p));
+        const double ct = trip(std::min(128, rows_p)), ck = per_k(std::min(128, rows_p), std::min(nb, cols_p));
         for (int x = ib + 1; x < ie; ++x)
-          if (pt[x - ib] + ck * pk[x - ib] + 1e-9 * per >= per * (double)cuts.size()) cuts.push_back(x);
+          if (ct * pt[x - ib] + ck * pk[x - ib] + 1e-9 * per >= per * (double)cuts.size()) cuts.push_back(x);
       }
       cuts.push_back(ie);
       // accumulation groups: of items with alpha = 1 (the first n1), broken
@@ -1824,7 +1883,7 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
           mma += 3.0 * 2.0 * 128 * tc_round16(hb) * pk.back();
           const Groups& G = groups_of(hb);
           const std::vector<int>& at = G.at;
-          const double ck = per_k(ha, hb);
+          const double ct = trip(ha), ck = per_k(ha, hb);
           t.bbeg = G.bbeg;
           t.bend = G.bend;
           int np = 0;
@@ -1844,7 +1903,7 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
             u.ibeg = at[c];
             u.iend = at[c + 1];
             const int x0 = u.ibeg - ib, x1 = u.iend - ib;
-            const double cost = pt[x1] - pt[x0] + ck * (pk[x1] - pk[x0]);
+            const double cost = ct * (pt[x1] - pt[x0]) + ck * (pk[x1] - pk[x0]);
             if (np <= 1) {
               u.direct = 1;
               u.out_off = S.offset;
@@ -1873,8 +1932,11 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
     }
   }
   std::vector<double> c1;
-  for (const TcTask& t : t1)
-    c1.push_back(item_cost(i1[t.ibeg], std::min(nb, t.b_rows - nb * t.tn)) + 200.0);
+  for (const TcTask& t : t1) {
+    const int hb = std::min(nb, t.b_rows - nb * t.tn);
+    c1.push_back(plan.tcx ? tcx_quarter_clocks(std::min(128, t.a_rows - 128 * t.tm)) + kTcxKClocks * hb * i1[t.ibeg].kp
+                          : item_cost(i1[t.ibeg], hb) + 200.0);
+  }
   laps.lap("phase-2 tasks");
   // tiles inside their operands (item shapes were checked against their
   // sectors when the items were made)
@@ -2022,34 +2084,37 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
     parallel_for((int)ranges.size(), [&](int j) {
       const int2& rg = ranges[j];
       int64_t pos = wr[j].x;
+      std::vector<int> rows, counts;
       for (int k = rg.x; k < rg.y; ++k) {
         const TcTask& T = tasks[order[k]];
-        TcxWork base{};
-        base.h_a = (int16_t)std::min(kTcRowsA, T.a_rows - kTcRowsA * T.tm);
-        base.h_b = (int16_t)std::min(nb, T.b_rows - nb * T.tn);
-        base.valid_rows = (int16_t)T.valid_rows;
-        base.valid_cols = (int16_t)T.valid_cols;
+        rows.push_back(std::min(kTcRowsA, T.a_rows - kTcRowsA * T.tm));
+        counts.push_back(std::max(1, T.iend - T.ibeg));
+      }
+      interleave_tasks(rows, counts, [&](int k, int at, int row0) {
+        const TcTask& T = tasks[order[rg.x + k]];
+        TcxWork x{};
+        x.h_a = (int16_t)rows[k];
+        x.h_b = (int16_t)std::min(nb, T.b_rows - nb * T.tn);
+        x.valid_rows = (int16_t)T.valid_rows;
+        x.valid_cols = (int16_t)T.valid_cols;
+        x.row0 = (uint8_t)row0;
         if (phase == 1) {
-          base.out_base = T.out_off / kTcxSlices + (int64_t)kTcRowsA * T.tm * T.out_kp;
-          base.out_ld = T.out_kp;
-          base.col0 = nb * T.tn;
+          x.out_base = T.out_off / kTcxSlices + (int64_t)kTcRowsA * T.tm * T.out_kp;
+          x.out_ld = T.out_kp;
+          x.col0 = nb * T.tn;
         } else if (T.direct) {
-          base.out_base = T.out_off + (int64_t)kTcRowsA * T.tm * T.out_kp + nb * T.tn;
-          base.out_ld = T.out_kp;
+          x.out_base = T.out_off + (int64_t)kTcRowsA * T.tm * T.out_kp + nb * T.tn;
+          x.out_ld = T.out_kp;
         } else {
-          base.out_base = T.out_off;
-          base.out_ld = base.h_b;
+          x.out_base = T.out_off;
+          x.out_ld = x.h_b;
         }
         const uint8_t f0 = (uint8_t)(T.direct ? kTcDirect : 0);
         if (T.ibeg == T.iend) {
-          TcxWork x = base;
           x.flags = (uint8_t)(f0 | kTcFirst | kTcLast | kTcEmpty);
-          w[pos++] = x;
-          continue;
-        }
-        for (int i = T.ibeg; i < T.iend; ++i) {
+        } else {
+          const int i = T.ibeg + at;
           const TcItem& it = items[i];
-          TcxWork x = base;
           x.a_base = it.a_off + (int64_t)kTcxSlices * kTcRowsA * T.tm * it.kp;
           x.b_base = it.b_off + (int64_t)kTcxSlices * nb * T.tn * it.kp;
           x.a_ex = it.a_ex + kTcRowsA * T.tm;
@@ -2059,10 +2124,10 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
           x.alpha = it.alpha64;
           x.a_pool = it.a_pool;
           x.b_pool = it.b_pool;
-          x.flags = (uint8_t)(f0 | (i == T.ibeg ? kTcFirst : 0) | (i + 1 == T.iend ? kTcLast : 0) | kTcGStart | kTcGEnd);
-          w[pos++] = x;
+          x.flags = (uint8_t)(f0 | (at == 0 ? kTcFirst : 0) | (i + 1 == T.iend ? kTcLast : 0) | kTcGStart | kTcGEnd);
         }
-      }
+        w[pos++] = x;
+      });
     });
   };
   std::vector<TcWork> w1, w2;
@@ -2331,7 +2396,7 @@ void GpuEngine::sigma_tcx(const Superblock& sb, SigmaPlan& p, const double* psi,
              "tcx T exponents");
   cuda_check(dev::launch_tcx_sigma(1, b, p.tcx_w1.d, p.tc_r1.d, (int)p.tc_r1.n, out, kWaitLimitNs, stream_),
              "tcx phase 1");
-  cuda_check(dev::launch_tcx_pack(b, p.tcx_tpack.d, (int)p.tcx_tpack.n, stream_), "tcx pack T");
+  cuda_check(dev::launch_tcx_pack(b, p.tcx_tpack.d, (int)p.tcx_tpack.n, stream_, p.tcx_t_split), "tcx pack T");
   cuda_check(dev::launch_tcx_sigma(2, b, p.tcx_w2.d, p.tc_r2.d, (int)p.tc_r2.n, out, kWaitLimitNs, stream_),
              "tcx phase 2");
   cuda_check(dev::launch_tcx_reduce(b, p.tc_tiles.d, p.tc_slots.d, (int)p.tc_tiles.n, out, stream_, p.tc_tile_split), "tcx reduce");
@@ -2442,7 +2507,7 @@ void GpuEngine::gemm_exact(const dev::Bufs& bufs, const std::vector<dev::GemmUni
       b.trans = g.tb ? 0 : 1;
       b.rows_v = u.n;
       b.cols_v = g.k;
-      b.rows_p = tc_round8(u.n);
+      b.rows_p = tc_round16(u.n);
       b.kp = tc_round16(g.k);
       b.rt = kTcxNB;
       b.pool = kTcPoolR;
@@ -2455,7 +2520,7 @@ void GpuEngine::gemm_exact(const dev::Bufs& bufs, const std::vector<dev::GemmUni
     }
   }
   if (ex_n[0] > INT32_MAX || ex_n[1] > INT32_MAX) throw std::runtime_error("gemm_exact: too many rows");
-  // tasks: 128 x 64 tiles of every unit, with the unit's items
+  // tasks: 128 x 32 tiles of every unit, with the unit's items
   struct Task {
     int u, tm, tn;
   };
@@ -2466,8 +2531,9 @@ void GpuEngine::gemm_exact(const dev::Bufs& bufs, const std::vector<dev::GemmUni
     for (int tm = 0; tm < (U.m + kTcRowsA - 1) / kTcRowsA; ++tm)
       for (int tn = 0; tn < (U.n + kTcxNB - 1) / kTcxNB; ++tn) {
         tasks.push_back({u, tm, tn});
+        const int ha = std::min(kTcRowsA, tc_round8(U.m) - kTcRowsA * tm), hb = std::min(kTcxNB, tc_round16(U.n) - kTcxNB * tn);
         double c = 400.0;
-        for (int i = U.ibeg; i < U.iend; ++i) c += 400.0 + tc_round16(items[i].k);
+        for (int i = U.ibeg; i < U.iend; ++i) c += tcx_quarter_clocks(ha) + kTcxKClocks * hb * tc_round16(items[i].k);
         cost.push_back(c);
       }
   }
@@ -2476,29 +2542,41 @@ void GpuEngine::gemm_exact(const dev::Bufs& bufs, const std::vector<dev::GemmUni
   std::vector<int> order;
   std::vector<int2> ranges;
   schedule_lpt(cost, bundle, tcx_blocks_per_sm() * sm_count(), order, ranges);
-  std::vector<TcxWork> w;
   std::vector<int2> wr(ranges.size());
+  int64_t nrec = 0;
   for (size_t j = 0; j < ranges.size(); ++j) {
-    wr[j].x = (int)w.size();
+    wr[j].x = (int)nrec;
+    for (int k = ranges[j].x; k < ranges[j].y; ++k)
+      nrec += std::max(1, units[tasks[order[k]].u].iend - units[tasks[order[k]].u].ibeg);
+    wr[j].y = (int)nrec;
+  }
+  if (nrec > INT32_MAX) throw std::runtime_error("gemm_exact: too many work records");
+  std::vector<TcxWork> w(nrec);
+  parallel_for((int)ranges.size(), [&](int j) {
+    int64_t pos = wr[j].x;
+    std::vector<int> rows, counts;
     for (int k = ranges[j].x; k < ranges[j].y; ++k) {
       const Task& T = tasks[order[k]];
       const GemmUnit& U = units[T.u];
-      TcxWork base{};
-      base.h_a = (int16_t)std::min(kTcRowsA, tc_round8(U.m) - kTcRowsA * T.tm);
-      base.h_b = (int16_t)std::min(kTcxNB, tc_round8(U.n) - kTcxNB * T.tn);
-      base.valid_rows = (int16_t)std::min(kTcRowsA, U.m - kTcRowsA * T.tm);
-      base.valid_cols = (int16_t)std::min(kTcxNB, U.n - kTcxNB * T.tn);
-      base.out_base = U.c_off + (int64_t)kTcRowsA * T.tm * U.ldc + kTcxNB * T.tn;
-      base.out_ld = U.ldc;
+      rows.push_back(std::min(kTcRowsA, tc_round8(U.m) - kTcRowsA * T.tm));
+      counts.push_back(std::max(1, U.iend - U.ibeg));
+    }
+    interleave_tasks(rows, counts, [&](int k, int at, int row0) {
+      const Task& T = tasks[order[ranges[j].x + k]];
+      const GemmUnit& U = units[T.u];
+      TcxWork x{};
+      x.h_a = (int16_t)rows[k];
+      x.h_b = (int16_t)std::min(kTcxNB, tc_round16(U.n) - kTcxNB * T.tn);
+      x.valid_rows = (int16_t)std::min(kTcRowsA, U.m - kTcRowsA * T.tm);
+      x.valid_cols = (int16_t)std::min(kTcxNB, U.n - kTcxNB * T.tn);
+      x.row0 = (uint8_t)row0;
+      x.out_base = U.c_off + (int64_t)kTcRowsA * T.tm * U.ldc + kTcxNB * T.tn;
+      x.out_ld = U.ldc;
       if (U.ibeg == U.iend) {
-        TcxWork x = base;
         x.flags = (uint8_t)(kTcDirect | kTcFirst | kTcLast | kTcEmpty);
-        w.push_back(x);
-        continue;
-      }
-      for (int i = U.ibeg; i < U.iend; ++i) {
+      } else {
+        const int i = U.ibeg + at;
         const GemmItem& g = items[i];
-        TcxWork x = base;
         const int kp = tc_round16(g.k);
         x.a_base = aref[i].off + (int64_t)kTcxSlices * kTcRowsA * T.tm * kp;
         x.b_base = bref[i].off + (int64_t)kTcxSlices * kTcxNB * T.tn * kp;
@@ -2508,13 +2586,11 @@ void GpuEngine::gemm_exact(const dev::Bufs& bufs, const std::vector<dev::GemmUni
         x.alpha = g.alpha;
         x.a_pool = kTcPoolL;
         x.b_pool = kTcPoolR;
-        x.flags = (uint8_t)(kTcDirect | (i == U.ibeg ? kTcFirst : 0) | (i + 1 == U.iend ? kTcLast : 0) |
-                            kTcGStart | kTcGEnd);
-        w.push_back(x);
+        x.flags = (uint8_t)(kTcDirect | (at == 0 ? kTcFirst : 0) | (i + 1 == U.iend ? kTcLast : 0) | kTcGStart | kTcGEnd);
       }
-    }
-    wr[j].y = (int)w.size();
-  }
+      w[pos++] = x;
+    });
+  });
   TcxBufs xb{};
   for (int i = 0; i < 4; ++i) xb.src[i] = bufs.p[i];
   __nv_bfloat16* pools[2] = {nullptr, nullptr};
@@ -2555,8 +2631,10 @@ void GpuEngine::gemm_exact(const dev::Bufs& bufs, const std::vector<dev::GemmUni
   xb.ex[kTcPoolR] = exs[1];
   xb.status = tc_status_;
   constexpr uint64_t kWaitLimitNs = 1000000000ull;
+  // blocks by the mean unit (see plan_tc)
+  const int split = (int)std::min<int64_t>(64, (pool_n[0] + pool_n[1]) / kTcxSlices / (2048 * (int64_t)packs.size()) + 1);
   cuda_check(launch_tcx_rowexp(xb, dp.d, (int)packs.size(), stream_), "exact gemm exponents");
-  cuda_check(launch_tcx_pack(xb, dp.d, (int)packs.size(), stream_), "exact gemm pack");
+  cuda_check(launch_tcx_pack(xb, dp.d, (int)packs.size(), stream_, split), "exact gemm pack");
   cuda_check(launch_tcx_sigma(2, xb, dw.d, dr.d, (int)wr.size(), bufs.p[c_buf], kWaitLimitNs, stream_),
              "exact gemm");
   dp.release(stream_);

@@ -145,6 +145,7 @@ struct SigmaPlan {
   double* tcx_t = nullptr;
   int64_t tcx_t_n = 0;
   DevArray<dev::TcPack> tcx_tpack;
+  int tcx_t_split = 1;  // blocks per unit of tcx_tpack
   DevArray<dev::TcxWork> tcx_w1, tcx_w2;
 };
 

@@ -197,14 +197,15 @@ cudaError_t launch_tc_reduce(const TcBufs& b, const TcTile* tiles, const int64_t
 // item) sum_q J_q 2^(7(5-q)) is formed exactly in int64 and added, times
 // alpha 2^(e_r + f_c - 49), to an FP64 accumulator of the output tile.
 // The pools hold six slices per block (tc_block_off times kTcxSlices; each
-// 16-column half of a block holds its six h x 16 slices together) and an
+// 16-column half of a block is one core-matrix operand of 6 h rows, slice after
+// slice; B operands have a multiple of 16 rows) and an
 // int32 row-exponent array each (the largest unbiased exponent of the row,
-// kTcxNoExp for a zero row).  Output tiles are 128 x 64.
+// kTcxNoExp for a zero row).  Output tiles are 128 x 32.
 constexpr int kTcxSlices = 6;
 constexpr int kTcxKBlock = 512;
 constexpr int kTcxKS = 16;  // K per pipeline stage (half of a K-chunk)
 constexpr int kTcxNoExp = -100000;
-constexpr int kTcxNB = kTcRowsB;
+constexpr int kTcxNB = 32;
 
 struct TcxBufs {
   const double* src[4];  // packing sources: L arena, R arena, psi, T (phase-1 output)
@@ -216,14 +217,15 @@ struct TcxBufs {
 };
 
 // One record of the exact kernels (80 bytes): as TcWork, with the FP64
-// alpha and the row-exponent offsets of A, B and (phase 1) of the T rows.
+// alpha, the row-exponent offsets of A, B and (phase 1) of the T rows, and the
+// first TMEM lane of the tile's rows (a multiple of 32; row0 + h_a <= 128).
 struct __align__(16) TcxWork {
   int64_t a_base, b_base, out_base;
   double alpha;
   int32_t kp, out_ld, col0;
   int32_t a_ex, b_ex, o_ex;
   int16_t h_a, h_b, valid_rows, valid_cols;
-  uint8_t a_pool, b_pool, flags, pad;
+  uint8_t a_pool, b_pool, flags, row0;
   int32_t pad2[3];
 };
 static_assert(sizeof(TcxWork) == 80, "TcxWork is 80 bytes");

@@ -12,11 +12,13 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def superblock(ctx, rows, cols, rng, nterms):
+def superblock(ctx, rows, cols, rng, nterms, sa=1.0, sb_=1.0):
     keys = np.array([[0, -1, -1, 0], [2, 0, 0, 0]], np.int32)  # HAM, CD(0,0;0): both rank 0
     hl, n = ctx.block_define([0], "c1", [[1, 1, 0]], [rows], keys)
     hr, m = ctx.block_define([0], "c1", [[1, 1, 0]], [cols], keys)
     A, B = rng.standard_normal((2, rows, rows)), rng.standard_normal((2, cols, cols))
+    A[1] *= sa
+    B[1] *= sb_
     ctx.block_upload(hl, A.reshape(-1))
     ctx.block_upload(hr, B.reshape(-1))
     ops = [(0, 0, -1, 0), (-1, 0, 0, 1)] + [(1, t % 2, 1, t // 2 % 2) for t in range(nterms)]
@@ -63,5 +65,40 @@ def test_exact_edges(gpu_ctx, rows, cols):
             ref = sigma(psi)
             got = gpu_ctx.sigma(sb, psi.reshape(-1)).reshape(rows, cols)
             assert np.linalg.norm(got - ref) <= 1e-11 * np.linalg.norm(ref), nterms
+    finally:
+        gpu_ctx.set_precision("fp64")
+
+
+# tiles of 1 to 4 lane quarters and 16 or 32 columns, K of 128 and 144 (two
+# ways to read the accumulators), of 512, 528 and 1040 (read-outs of 512)
+@pytest.mark.parametrize("rows,cols", [(32, 33), (33, 16), (96, 31), (97, 128), (129, 144), (40, 512), (520, 24), (1030, 530)])
+def test_exact_tiles_and_blocks(gpu_ctx, rows, cols):
+    rng = np.random.default_rng(1000 * rows + cols)
+    try:
+        gpu_ctx.set_precision("exacttc")
+        for nterms in (1, 7):
+            sb, sigma = superblock(gpu_ctx, rows, cols, rng, nterms)
+            psi = rng.standard_normal((rows, cols))
+            ref = sigma(psi)
+            for _ in range(2):
+                got = gpu_ctx.sigma(sb, psi.reshape(-1)).reshape(rows, cols)
+                assert np.linalg.norm(got - ref) <= 1e-11 * np.linalg.norm(ref), nterms
+    finally:
+        gpu_ctx.set_precision("fp64")
+
+
+# scales of the products out of the range of one power of two
+@pytest.mark.parametrize("ea,eb,ep", [(500, -500, 0), (510, -500, 505), (-480, 490, -470), (300, 200, 460)])
+def test_exact_far_scales(gpu_ctx, ea, eb, ep):
+    rng = np.random.default_rng(7)
+    try:
+        gpu_ctx.set_precision("exacttc")
+        sb, sigma = superblock(gpu_ctx, 21, 19, rng, 4, 2.0**ea, 2.0**eb)
+        psi = 2.0**ep * rng.standard_normal((21, 19))
+        ref = sigma(psi)
+        got = gpu_ctx.sigma(sb, psi.reshape(-1)).reshape(21, 19)
+        assert np.isfinite(ref).all()
+        big = np.abs(ref).max()
+        assert np.linalg.norm((got - ref) / big) <= 1e-11 * np.linalg.norm(ref / big)
     finally:
         gpu_ctx.set_precision("fp64")
