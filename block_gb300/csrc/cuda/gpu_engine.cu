@@ -1294,10 +1294,11 @@ void GpuEngine::plan_tc(const Superblock& sb, SigmaPlan& plan) {
   std::unordered_map<int64_t, int> lmap, rmap;  // (block offset, transposed) -> index in ops_packs
   lmap.reserve(1 << 16);
   rmap.reserve(1 << 16);
+  int last_pack = -1;  // index in ops_packs of the unit returned last
   auto pack_view = [&](int pool, const HostView& v, std::unordered_map<int64_t, int>& m) -> TcPack {
     const int64_t key = v.off * 2 + (v.trans ? 1 : 0);
     auto it = m.find(key);
-    if (it != m.end()) return ops_packs[it->second];
+    if (it != m.end()) return ops_packs[last_pack = it->second];
     TcPack p{};
     p.src_off = v.off;
     p.ld = v.ld;
@@ -1313,7 +1314,8 @@ void GpuEngine::plan_tc(const Superblock& sb, SigmaPlan& plan) {
     pool_n[pool] += nsl * (int64_t)p.rows_p * p.kp;  // all slices
     p.ex_off = (int32_t)ex_n[pool];
     ex_n[pool] += p.rows_p;
-    m.emplace(key, (int)ops_packs.size());
+    last_pack = (int)ops_packs.size();
+    m.emplace(key, last_pack);
     ops_packs.push_back(p);
     return p;
   };
@@ -1352,6 +1354,7 @@ void GpuEngine::plan_tc(const Superblock& sb, SigmaPlan& plan) {
   }
   std::vector<TcItem> i1;
   std::vector<TcTask> t1;
+  std::vector<int> i1_pack;       // pack unit of each stage-1 item's operator
   std::vector<int> sec1;          // psi sector read by each phase-1 task
   std::vector<int64_t> bundle1;  // tasks reading the same A row tile
   std::vector<std::vector<TcItem>> per_sector(nsec);
@@ -1445,6 +1448,7 @@ void GpuEngine::plan_tc(const Superblock& sb, SigmaPlan& plan) {
           fail();
         const int idx = (int)i1.size();
         i1.push_back(a);
+        i1_pack.push_back(last_pack);
         for (int tm = 0; tm < (mr + 127) / 128; ++tm)
           for (int tn = 0; tn < (mc + nb - 1) / nb; ++tn) {
             TcTask t{};
@@ -1519,33 +1523,32 @@ void GpuEngine::plan_tc(const Superblock& sb, SigmaPlan& plan) {
   std::vector<TcRow> rows_tab;
   int64_t n_stacks = 0, n_stacked = 0;
   if (!plan.tcx && tc_stack_rows > 0) {
-    std::unordered_map<int64_t, int> lpack;  // pool-L offset -> its pack unit
-    for (size_t i = 0; i < ops_packs.size(); ++i)
-      if (ops_packs[i].pool == kTcPoolL) lpack.emplace(ops_packs[i].dst_off, (int)i);
+    // an item's tasks follow one another: first[u] .. first[u + 1]
     const size_t ni = i1.size();
-    std::vector<std::vector<int>> tasks_of(ni);
-    for (size_t k = 0; k < t1.size(); ++k) tasks_of[t1[k].ibeg].push_back((int)k);
+    std::vector<int> first(ni + 1, 0);
+    for (const TcTask& t : t1) ++first[t.ibeg + 1];
+    for (size_t u = 0; u < ni; ++u) first[u + 1] += first[u];
     auto task_mma = [&](const TcTask& t) {
       return 3.0 * 2.0 * 128 * tc_round16(std::min(nb, t.b_rows - nb * t.tn)) * i1[t.ibeg].kp;
     };
-    // candidates grouped by (psi^T block, K), each group in item order
-    std::map<std::pair<int64_t, int>, std::vector<int>> groups;
+    // candidates grouped by psi sector (which gives the psi^T block and K), each
+    // group in item order
+    std::vector<std::vector<int>> groups(nsec);
     for (size_t u = 0; u < ni; ++u) {
-      if (tasks_of[u].empty() || i1[u].a_pool != kTcPoolL) continue;
-      if (t1[tasks_of[u][0]].a_rows > std::min(tc_stack_rows, kTcRowsA)) continue;
-      groups[{i1[u].b_off, i1[u].kp}].push_back((int)u);
+      if (first[u] == first[u + 1] || i1[u].a_pool != kTcPoolL) continue;
+      if (t1[first[u]].a_rows > std::min(tc_stack_rows, kTcRowsA)) continue;
+      groups[sec1[first[u]]].push_back((int)u);
     }
     std::vector<char> drop(t1.size(), 0);
     std::vector<TcTask> t_new;
     std::vector<int> sec_new;
     std::vector<int64_t> bun_new;
-    for (const auto& g : groups) {
-      const std::vector<int>& us = g.second;
+    for (const std::vector<int>& us : groups) {
       size_t x = 0;
       while (x < us.size()) {
         size_t y = x;
         int H = 0;
-        while (y < us.size() && H + t1[tasks_of[us[y]][0]].a_rows <= kTcRowsA) H += t1[tasks_of[us[y++]][0]].a_rows;
+        while (y < us.size() && H + t1[first[us[y]]].a_rows <= kTcRowsA) H += t1[first[us[y++]]].a_rows;
         if (y - x < 2) {
           x = y;
           continue;
@@ -1558,17 +1561,16 @@ void GpuEngine::plan_tc(const Superblock& sb, SigmaPlan& plan) {
         int r0 = 0;
         for (size_t m = x; m < y; ++m) {
           const int u = us[m];
-          const TcTask& T = t1[tasks_of[u][0]];
-          auto it = lpack.find(i1[u].a_off);
-          if (it == lpack.end() || i1[u].kp != kp || T.tm != 0) fail();
-          TcPack pk = ops_packs[it->second];
+          const TcTask& T = t1[first[u]];
+          TcPack pk = ops_packs[i1_pack[u]];
+          if (pk.pool != kTcPoolL || pk.dst_off != i1[u].a_off || i1[u].kp != kp || i1[u].b_off != i1[us[x]].b_off || T.tm != 0) fail();
           pk.dst_off = st_off;
           pk.row0 = r0;
           pk.dst_rows = H;
           ops_packs.push_back(pk);
           for (int lr = 0; lr < T.a_rows; ++lr)
             rows_tab[base + r0 + lr] = TcRow{T.out_off, (int16_t)T.a_rows, (int16_t)lr, i1[u].alpha};
-          for (int k : tasks_of[u]) {
+          for (int k = first[u]; k < first[u + 1]; ++k) {
             drop[k] = 1;
             mma -= task_mma(t1[k]);
           }
@@ -1580,7 +1582,7 @@ void GpuEngine::plan_tc(const Superblock& sb, SigmaPlan& plan) {
         si.alpha64 = 1.0;
         const int idx = (int)i1.size();
         i1.push_back(si);
-        for (int k : tasks_of[us[x]]) {
+        for (int k = first[us[x]]; k < first[us[x] + 1]; ++k) {
           TcTask t = t1[k];
           t.a_rows = H;
           t.ibeg = idx;
