@@ -5,8 +5,10 @@
 // tridiagonal form followed by the implicit QL/QR iteration with the
 // accumulated rotations.  This is the same family of algorithm, laid out
 // for the GPU:
-//   1. Householder tridiagonalisation, two launches per column step for all
-//      sectors at once: a per-sector "house" kernel forms the reflector of
+//   1. Householder tridiagonalisation: a sector of order up to eig_cluster_max_n()
+//      stays in the shared memory of one thread-block cluster for all its
+//      columns (eig_tridiag_cluster, k_eig.cu).  Larger sectors take two launches
+//      per column step, all at once: a per-sector "house" kernel forms the reflector of
 //      column k from a lazily corrected copy of that column, and a tiled
 //      "update" kernel applies the previous step's rank-2 update to the lower
 //      triangle of the trailing matrix and, in the same pass, forms the
