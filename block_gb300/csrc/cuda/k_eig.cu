@@ -302,8 +302,16 @@ __global__ void __launch_bounds__(kBtThreads) eig_backtransform(EigBufs b, const
 constexpr int kClThreads = 512, kClWarps = kClThreads / 32;
 constexpr int kClSumWarps = 4;
 
-__device__ __forceinline__ void cl_arrive() { __syncwarp(); asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// (.aligned: every lane of a warp executes them together, also behind a loop that
+// the lanes leave after different numbers of turns)
+__device__ __forceinline__ void cl_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cl_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ uint32_t cl_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
