@@ -32,16 +32,6 @@ __device__ __forceinline__ double warp_max(double x) {
   return x;
 }
 
-// h^-1/2 for normal h: the hardware's approximation y (relative error below
-// 2^-20), then y (1 - r)^-1/2 with r = 1 - h y^2 by the binomial series to
-// second order (error 5 r^3 / 16 below 2^-60 before rounding)
-__device__ __forceinline__ double inv_sqrt(double h) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(h));
-  const double r = fma(-h * y, y, 1.0);
-  return fma(y * r, fma(0.375, r, 0.5), y);
-}
-
 // scalar work area of a job (k_eig.cu): d, e, tau, unsorted eigenvalues, ...
 __device__ __forceinline__ double* diag_of(double* work, const EigJob& J) { return work + J.s_off; }
 __device__ __forceinline__ double* offd_of(double* work, const EigJob& J) { return work + J.s_off + J.n; }
@@ -77,10 +67,9 @@ __global__ void dc_tear_kernel(double* work, const EigJob* __restrict__ jobs, co
 // every lane applies them to its row of the leaf's Z.
 // Bound by the recurrence: one thread's FP64 operations issue every 63
 // clocks, so their number counts.  The leaf is scaled by a power of two to
-// norm near one, so that the rotation comes from one reciprocal square root
-// of f^2 + g^2 (about 20 operations a rotation instead of about 60 with
-// hypot and two divisions; leaves of the 12 matrices up to order 400:
-// 1973 -> 1095 us).
+// norm near one, so that the rotation comes from one rsqrt() of f^2 + g^2
+// instead of hypot and two divisions (leaves of the 12 matrices up to order
+// 400: 1973 -> about 1100 us).
 __global__ void __launch_bounds__(32 * kLeafWarps) dc_leaf_kernel(double* work, const EigJob* __restrict__ jobs,
                                                                   const DcLeaf* __restrict__ leaves, int nleaves,
                                                                   int* status) {
@@ -151,7 +140,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps) dc_leaf_kernel(double* work, 
             early = true;
             break;
           }
-          const double q = inv_sqrt(h);
+          const double q = rsqrt(h);
           e[i + 1] = h * q;
           s = f * q;
           c = g * q;
