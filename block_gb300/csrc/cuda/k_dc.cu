@@ -598,8 +598,13 @@ cudaError_t launch_dc_deflate(double* work, const EigJob* jobs, const DcLevel& L
   if (max_nm < 2 || max_nm > kEigMaxN) return cudaErrorInvalidValue;
   int P = 1;
   while (P < max_nm) P <<= 1;
-  const size_t smem = (size_t)P * (3 * sizeof(double) + 2 * sizeof(int));
-  cudaError_t e = cudaFuncSetAttribute(dc_deflate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  constexpr size_t per_pole = 3 * sizeof(double) + 2 * sizeof(int);
+  static_assert((kEigMaxN & (kEigMaxN - 1)) == 0, "P is at most kEigMaxN");
+  const size_t smem = per_pole * P;
+  // the same limit for every call: another context's thread may set it between
+  // here and the launch
+  cudaError_t e = cudaFuncSetAttribute(dc_deflate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(per_pole * kEigMaxN));
   if (e != cudaSuccess) return e;
   dc_deflate_kernel<<<L.nmerges, kDefThreads, smem, s>>>(work, jobs, L);
   return cudaGetLastError();

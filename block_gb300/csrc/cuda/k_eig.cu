@@ -578,7 +578,10 @@ cudaError_t launch_eig_tridiag_cluster(const EigBufs& b, const EigJob* jobs, con
   if (dims[0] < 1 || dims[0] > eig_cluster_max_n()) return cudaErrorInvalidValue;
   const int c = eig_cluster_size(dims, njobs);
   const size_t smem = cl_smem(dims[0], c);
-  cudaError_t e = cudaFuncSetAttribute(eig_tridiag_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the kernel's limits are always set to the same values: another context's thread
+  // may set them between here and the launch
+  cudaError_t e =
+      cudaFuncSetAttribute(eig_tridiag_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClSmemMax);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(eig_tridiag_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
@@ -603,8 +606,10 @@ cudaError_t launch_eig_backtransform(const EigBufs& b, const EigJob* jobs, int n
                                      cudaStream_t s) {
   if (njobs <= 0) return cudaSuccess;
   if (max_n < 1 || max_n > kEigMaxN) return cudaErrorInvalidValue;
-  const size_t smem = (size_t)(2 + kEigBtCols) * max_n * sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(eig_backtransform, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  constexpr size_t per_row = (2 + kEigBtCols) * sizeof(double);
+  const size_t smem = per_row * max_n;
+  cudaError_t e = cudaFuncSetAttribute(eig_backtransform, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(per_row * kEigMaxN));  // as above: the same for every call
   if (e != cudaSuccess) return e;
   eig_backtransform<<<bt_ctas, kBtThreads, smem, s>>>(b, jobs, njobs, max_n);
   return cudaGetLastError();

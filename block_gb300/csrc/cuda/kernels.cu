@@ -549,9 +549,12 @@ cudaError_t launch_jacobi(double* A, const int64_t* a_off, const int* dims, doub
   if (nmat <= 0) return cudaSuccess;
   const int m = max_n + (max_n & 1);
   const size_t smem = (size_t)(m / 2) * (2 * sizeof(double) + 2 * sizeof(int)) + 16;
-  if (smem > 200 * 1024) return cudaErrorInvalidValue;
+  constexpr size_t kMost = 200 * 1024;
+  if (smem > kMost) return cudaErrorInvalidValue;
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the same limit for every call: another context's thread may set it between
+    // here and the launch
+    cudaError_t e = cudaFuncSetAttribute(jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost);
     if (e != cudaSuccess) return e;
   }
   jacobi_kernel<<<nmat, 512, smem, s>>>(A, a_off, dims, w, w_off, V, v_off, status);
