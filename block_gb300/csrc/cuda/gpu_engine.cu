@@ -4068,18 +4068,32 @@ int* GpuEngine::eigh_batched(const std::vector<int>& dims, double* a, const std:
   dj.upload(jobs, stream_);
   dev::EigBufs eb{copy_inputs ? wk : a, z, w, wk, status};
   // The jobs by descending order: the largest start first in the
-  // tridiagonalisation (orders that fit a cluster's shared memory in one
-  // launch, the larger ones with two launches a column) and in the
-  // back-transformation.
+  // tridiagonalisation (orders that fit a cluster's shared memory in a launch or
+  // a few, the larger ones with two launches a column) and in the
+  // back-transformation.  The others ride along in the larger ones' launches
+  // where the tiles of all fit the SMs at once: they cost next to nothing there
+  // (orders 700 and 5 of 200: 18.3 ms, 19.7 with clusters behind; 1000 and 200 of
+  // 100, which do not fit: 36.2, 30.8 with clusters).
   std::vector<dev::EigJob> sorted = jobs;
   std::stable_sort(sorted.begin(), sorted.end(), [](const dev::EigJob& x, const dev::EigJob& y) { return x.n > y.n; });
+  if (!eig_clusters_known_) {
+    cuda_check(dev::eig_clusters(eig_clusters_), "eigensolver clusters");
+    eig_clusters_known_ = true;
+  }
+  const int cluster_n = dev::eig_cluster_max_n(eig_clusters_);
   int nbig = 0;
+  int64_t all_tiles = 0;
+  for (const dev::EigJob& J : sorted) {
+    all_tiles += J.nt * (J.nt + 1) / 2;
+    if (J.n > cluster_n) ++nbig;
+  }
+  if (nbig > 0 && all_tiles <= sm_count()) nbig = nj;
   std::vector<int> small_n;
-  for (dev::EigJob& J : sorted) {
-    if (J.n > dev::eig_cluster_max_n()) {
+  for (int j = 0; j < nj; ++j) {
+    dev::EigJob& J = sorted[j];
+    if (j < nbig) {
       J.tile0 = tiles;
       tiles += J.nt * (J.nt + 1) / 2;
-      ++nbig;
     } else {
       small_n.push_back(J.n);
     }
@@ -4089,8 +4103,12 @@ int* GpuEngine::eigh_batched(const std::vector<int>& dims, double* a, const std:
   DevArray<dev::EigJob> dsorted;
   dsorted.upload(sorted, stream_);
   cuda_check(dev::launch_eig_tridiag(eb, dsorted.d, nbig, max_n, tiles, stream_), "eigensolver tridiagonalisation");
-  cuda_check(dev::launch_eig_tridiag_cluster(eb, dsorted.d + nbig, small_n.data(), nj - nbig, stream_),
-             "eigensolver tridiagonalisation (clusters)");
+  int at = 0;
+  for (const dev::EigClass& c : dev::eig_cluster_classes(eig_clusters_, small_n.data(), nj - nbig)) {
+    cuda_check(dev::launch_eig_tridiag_cluster(eb, dsorted.d + nbig + at, small_n[at], c, stream_),
+               "eigensolver tridiagonalisation (clusters)");
+    at += c.jobs;
+  }
   tridiagonal_dc(jobs, dj.d, wk, status);
   cuda_check(dev::launch_eig_backtransform(eb, dsorted.d, nj, max_n, bt, stream_), "eigensolver back-transformation");
   dj.release(stream_);

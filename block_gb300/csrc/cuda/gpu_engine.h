@@ -363,6 +363,9 @@ class GpuEngine : public Engine {
   // second stream (density): forked from and joined to stream_ within a call
   cudaStream_t side_stream_ = nullptr;
   cudaEvent_t side_fork_ = nullptr, side_join_ = nullptr;
+  // thread-block clusters of the eigensolver on this device, asked for once
+  dev::EigClusters eig_clusters_{};
+  bool eig_clusters_known_ = false;
   // rotation that made each renormalised block (big-block quantum q: n[q] x m[q]
   // row-major at off[q]), kept for the wavefunction guess transform
   struct RotRecord {

@@ -547,37 +547,15 @@ size_t cl_smem(int n, int c) { return ((size_t)4 * n + (size_t)((n + c - 1) / c)
 constexpr size_t kClSmemMax = 226 * 1024;
 }  // namespace
 
-int eig_cluster_max_n() {
+// largest order that clusters of 1 << k blocks hold
+static int eig_cluster_order(int k) {
   int n = 1;
-  while (cl_smem(n + 1, 16) <= kClSmemMax) ++n;
+  while (cl_smem(n + 1, 1 << k) <= kClSmemMax) ++n;
   return n;
 }
 
-// Cluster size for a batch (orders in descending order): 8 blocks (15 such
-// clusters fit the GPU) or 16 (7 clusters, for orders whose matrix needs
-// them or whose FP64 work decides), by the time of the jobs dealt to the free
-// clusters in order; a job takes n^3 / 1.7 C clocks of FMAs and about 5000 a
-// column for the exchanges and scalars.
-static int eig_cluster_size(const int* dims, int njobs) {
-  auto makespan = [&](int c, int slots) {
-    std::vector<double> t(std::min(slots, njobs), 0.0);
-    for (int j = 0; j < njobs; ++j) {
-      const double n = dims[j];
-      *std::min_element(t.begin(), t.end()) += n * n * n / (1.7 * c) + 5000.0 * n;
-    }
-    return *std::max_element(t.begin(), t.end());
-  };
-  const int n = dims[0];
-  if (cl_smem(n, 8) > kClSmemMax) return 16;
-  return makespan(16, 7) < makespan(8, 15) ? 16 : 8;
-}
-
-cudaError_t launch_eig_tridiag_cluster(const EigBufs& b, const EigJob* jobs, const int* dims, int njobs,
-                                       cudaStream_t s) {
-  if (njobs <= 0) return cudaSuccess;
-  if (dims[0] < 1 || dims[0] > eig_cluster_max_n()) return cudaErrorInvalidValue;
-  const int c = eig_cluster_size(dims, njobs);
-  const size_t smem = cl_smem(dims[0], c);
+static cudaError_t eig_cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, int c, int nclusters,
+                                      size_t smem, cudaStream_t s) {
   // the kernel's limits are always set to the same values: another context's thread
   // may set them between here and the launch
   cudaError_t e =
@@ -585,18 +563,108 @@ cudaError_t launch_eig_tridiag_cluster(const EigBufs& b, const EigJob* jobs, con
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(eig_tridiag_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(c * njobs));
+  cfg = {};
+  cfg.gridDim = dim3((unsigned)(c * nclusters));
   cfg.blockDim = dim3(kClThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)c;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
+  attr = {};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)c;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
   cfg.numAttrs = 1;
+  return cudaSuccess;
+}
+
+cudaError_t eig_clusters(EigClusters& ec) {
+  for (int k = 0; k < kEigClusterSizes; ++k) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    const cudaError_t e = eig_cluster_config(cfg, attr, 1 << k, 1, kClSmemMax, nullptr);
+    if (e != cudaSuccess) return e;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, eig_tridiag_cluster, &cfg) != cudaSuccess) {
+      cudaGetLastError();  // no cluster of this size
+      n = 0;
+    }
+    ec.resident[k] = n;
+    ec.order[k] = n > 0 ? eig_cluster_order(k) : 0;
+  }
+  return cudaSuccess;
+}
+
+int eig_cluster_max_n(const EigClusters& ec) { return *std::max_element(ec.order, ec.order + kEigClusterSizes); }
+
+// Orders fall into classes by the smallest clusters that hold them; runs of
+// neighbouring classes share a launch, and each launch takes the cluster size
+// with which it ends first: small clusters for many matrices (400 of order 100:
+// 2.1 ms with one block each, 11.9 with 8, 7.0 with the tiled launches), large
+// ones for few (12 up to order 400: 2.9 ms with 16 blocks, 3.8 with 8).  A job
+// takes n^3 / 1.7 C clocks of FMAs and 7400 + 90 C a column for the exchanges and
+// scalars (fitted to orders 100 to 640).  The jobs of a launch, in descending
+// order, run as clusters become free: their time lies between their sum over
+// the resident clusters and that of rounds of the largest jobs.  The launches run
+// one after the other.
+std::vector<EigClass> eig_cluster_classes(const EigClusters& ec, const int* dims, int njobs) {
+  if (njobs <= 0) return {};
+  std::vector<int> at{0};  // first jobs of the classes
+  auto needs = [&](int n) {
+    int k = 0;
+    while (k < kEigClusterSizes && ec.order[k] < n) ++k;
+    return k;
+  };
+  std::vector<double> s1(njobs + 1, 0.0), s3(njobs + 1, 0.0);
+  for (int j = 0; j < njobs; ++j) {
+    const double n = dims[j];
+    s1[j + 1] = s1[j] + n;
+    s3[j + 1] = s3[j] + n * n * n;
+    if (j > 0 && needs(dims[j]) != needs(dims[j - 1])) at.push_back(j);
+  }
+  at.push_back(njobs);
+  const int nc = (int)at.size() - 1;
+  std::vector<double> best(nc + 1, 1e300);
+  std::vector<EigClass> last(nc + 1);
+  best[0] = 0.0;
+  for (int i = 0; i < nc; ++i)
+    for (int k = 0; k < kEigClusterSizes; ++k) {
+      if (ec.order[k] < dims[at[i]]) continue;
+      const double fma = 1.0 / (1.7 * (1 << k)), col = 7400.0 + 90.0 * (1 << k);
+      for (int e = i + 1; e <= nc; ++e) {
+        double rounds = 0.0;
+        for (int j = at[i]; j < at[e]; j += ec.resident[k]) {
+          const double n = dims[j];
+          rounds += n * n * n * fma + n * col;
+        }
+        const double n0 = dims[at[i]], one = n0 * n0 * n0 * fma + n0 * col;
+        const double even = ((s3[at[e]] - s3[at[i]]) * fma + (s1[at[e]] - s1[at[i]]) * col) / ec.resident[k];
+        const double t = best[i] + 0.5 * (rounds + std::max(one, even));
+        if (t < best[e]) {
+          best[e] = t;
+          last[e] = {at[e] - at[i], k};
+        }
+      }
+    }
+  std::vector<EigClass> out;
+  for (int e = nc; e > 0;) {
+    out.push_back(last[e]);
+    const int first = at[e] - last[e].jobs;
+    while (at[e] != first) --e;
+  }
+  std::reverse(out.begin(), out.end());
+  return out;
+}
+
+cudaError_t launch_eig_tridiag_cluster(const EigBufs& b, const EigJob* jobs, int max_n, const EigClass& cl,
+                                       cudaStream_t s) {
+  if (cl.jobs <= 0) return cudaSuccess;
+  if (cl.k < 0 || cl.k >= kEigClusterSizes || max_n < 1 || cl_smem(max_n, 1 << cl.k) > kClSmemMax)
+    return cudaErrorInvalidValue;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr;
+  cudaError_t e = eig_cluster_config(cfg, attr, 1 << cl.k, cl.jobs, cl_smem(max_n, 1 << cl.k), s);
+  if (e != cudaSuccess) return e;
   e = cudaLaunchKernelEx(&cfg, eig_tridiag_cluster, b, jobs);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
@@ -609,7 +677,7 @@ cudaError_t launch_eig_backtransform(const EigBufs& b, const EigJob* jobs, int n
   constexpr size_t per_row = (2 + kEigBtCols) * sizeof(double);
   const size_t smem = per_row * max_n;
   cudaError_t e = cudaFuncSetAttribute(eig_backtransform, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(per_row * kEigMaxN));  // as above: the same for every call
+                                       (int)(per_row * kEigMaxN));  // the same for every call, as above
   if (e != cudaSuccess) return e;
   eig_backtransform<<<bt_ctas, kBtThreads, smem, s>>>(b, jobs, njobs, max_n);
   return cudaGetLastError();

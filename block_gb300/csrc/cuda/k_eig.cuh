@@ -5,7 +5,7 @@
 // tridiagonal form followed by the implicit QL/QR iteration with the
 // accumulated rotations.  This is the same family of algorithm, laid out
 // for the GPU:
-//   1. Householder tridiagonalisation: a sector of order up to eig_cluster_max_n()
+//   1. Householder tridiagonalisation: a sector of order up to 641 (16 blocks)
 //      stays in the shared memory of one thread-block cluster for all its
 //      columns (eig_tridiag_cluster, k_eig.cu).  Larger sectors take two launches
 //      per column step, all at once: a per-sector "house" kernel forms the reflector of
@@ -26,6 +26,7 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <vector>
 
 namespace bgpu {
 namespace dev {
@@ -67,11 +68,24 @@ struct EigBufs {
 };
 cudaError_t launch_eig_tridiag(const EigBufs& b, const EigJob* jobs, int njobs, int max_n, int tiles,
                                cudaStream_t s);
-// The same for matrices of order at most eig_cluster_max_n(), each held in the
-// shared memory of a thread-block cluster, in one launch; dims (host): the
-// jobs' orders, in descending order.
-int eig_cluster_max_n();
-cudaError_t launch_eig_tridiag_cluster(const EigBufs& b, const EigJob* jobs, const int* dims, int njobs,
+// The same for matrices each held in the shared memory of a thread-block
+// cluster of 1 << k blocks.
+constexpr int kEigClusterSizes = 5;
+struct EigClusters {
+  int resident[kEigClusterSizes];  // clusters of 1 << k blocks that the device runs at once (0: none can be placed)
+  int order[kEigClusterSizes];     // largest order that they hold (0: none)
+};
+cudaError_t eig_clusters(EigClusters& ec);
+// largest order that any of them holds (0: no clusters)
+int eig_cluster_max_n(const EigClusters& ec);
+struct EigClass {
+  int jobs, k;
+};
+// Jobs of orders dims (host, in descending order, at most eig_cluster_max_n) cut
+// into launches: the next `jobs` of them on clusters of 1 << k blocks.
+std::vector<EigClass> eig_cluster_classes(const EigClusters& ec, const int* dims, int njobs);
+// one of these launches; max_n: its first (largest) order
+cudaError_t launch_eig_tridiag_cluster(const EigBufs& b, const EigJob* jobs, int max_n, const EigClass& cl,
                                        cudaStream_t s);
 // Eigenvector signs made canonical: in matrix q (order dims[q] at V +
 // off[q], eigenvectors as columns, column-major when colmajor[q] else

@@ -107,3 +107,26 @@ def test_batch_larger_than_the_resident_clusters(gpu_ctx):
         mats.append(0.5 * (X + X.T))
     for A, (w, V) in zip(mats, gpu_ctx.diagonalise(mats)):
         check(A, w, V)
+
+
+@pytest.mark.parametrize("orders", [
+    [100] * 180 + [167, 168, 235, 236],  # one-block clusters in two rounds, the largest that 1 and 2 blocks hold
+    [331, 332, 464, 465, 641] + [40] * 20 + [165, 166],  # every class, each with its own launch or shared
+    [700, 200, 150, 5],  # all in the tiled launches
+    [650] + [90] * 60 + [300],  # tiled, then clusters
+], ids=["many", "classes", "ride", "behind"])
+def test_batches_across_the_cluster_classes(gpu_ctx, orders):
+    """Batches cut into launches of several cluster sizes; the same bits as
+    each matrix gives in a batch of equals where both run on clusters."""
+    rng = np.random.default_rng(len(orders))
+    mats = []
+    for n in orders:
+        X = rng.standard_normal((n, n))
+        mats.append(0.5 * (X + X.T))
+    got = gpu_ctx.diagonalise(mats)
+    for A, (w, V) in list(zip(mats, got))[:: max(1, len(orders) // 24)]:
+        check(A, w, V)
+    if max(orders) <= 641:
+        for i in (0, len(orders) - 1):
+            (w, V), = gpu_ctx.diagonalise([mats[i]])
+            assert np.array_equal(w, got[i][0]) and np.array_equal(V, got[i][1])
