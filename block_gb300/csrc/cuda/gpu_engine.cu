@@ -1717,9 +1717,10 @@ TcKnobs GpuEngine::tc_default_knobs() const {
 }
 
 // Phase-2 tasks, cost model, block assignment and flattened work records of
-// a tensor-core plan for one set of knobs.  Persistent schedule: two blocks
-// per SM, longest-processing-time assignment; tiles costing more than
-// total / (2 split SMs) are cut into pieces summed by the reduce kernel.
+// a tensor-core plan for one set of knobs.  Persistent schedule: phase 1 by
+// longest processing time, phase 2 in the order of its pieces (schedule_list);
+// sectors whose tiles cost more than a 2 split-th of a block's share are cut
+// into pieces summed by the reduce kernel.
 // Per-sector schedule (baseline): no cut tiles, one block per task, one
 // launch per psi sector (phase 1) and per sigma sector (phase 2).
 void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs& kn) {
@@ -1745,7 +1746,7 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
   std::vector<TcTile> tiles;
   std::vector<int64_t> slots;
   auto round_cols = [&](int x) { return plan.tcx ? tc_round16(x) : tc_round8(x); };  // as packed (plan_tc)
-  std::vector<int> breaks;  // per tile: items at which an accumulation group starts anew
+  std::vector<int> breaks;  // per tile width of a sector: items at which an accumulation group starts anew
   const int group_items = std::max(1, kn.group);
   constexpr int kGroupK = 1024;
   int64_t partial_n = 0;
@@ -1761,28 +1762,27 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
   {
     // Clocks of an item of a tile: its MMAs (three per K=16 step, each reading
     // 128 rows of A and the columns of B from shared memory at 128 bytes a
-    // clock), the trips through the pipeline of the item and of its pieces
-    // of 64 K, and a little for its bytes (fitted to the blocks' clocks at
-    // 24 orbitals M=500 and 18 orbitals M=1000, 1 % rms; by K times columns
-    // alone the slowest block took 1.4 times the mean).
+    // clock), the trips through the pipeline of the item (0.35 of the item_cost
+    // knob: 140) and of its pieces of 64 K, and a little for its bytes (fitted to
+    // the blocks' clocks at 24 orbitals M=500 and 18 orbitals M=1000, 1 % rms; by
+    // K times columns alone the slowest block took 1.4 times the mean).
     // Sums over items of a sector come from prefix sums of what does not
     // depend on the tile (trips) and of K.
     // The exact kernels' items cost their quarters of rows and their K times
-    // columns (tcx_quarter_clocks, tcx_k_clocks).
+    // columns (tcx_quarter_clocks, kTcxKClocks).
     const double mma_step = 3.0 / 16.0;
-    auto trips = [&](const TcItem& it) { return plan.tcx ? 1.0 : 140.0 + 250.0 * ((it.kp + 63) / 64); };
+    auto trips = [&](const TcItem& it) { return plan.tcx ? 1.0 : 0.35 * kn.item_cost + 250.0 * ((it.kp + 63) / 64); };
     auto trip = [&](int ha) { return plan.tcx ? tcx_quarter_clocks(ha) : 1.0; };
     auto per_k = [&](int ha, int hb) {
       return plan.tcx ? kTcxKClocks * hb : mma_step * (32.0 + tc_round16(hb) / 4.0) + 0.016 * (ha + hb);
     };
     // Pieces: every tile of a sector is cut at about the same items, into
-    // pieces of at most a kPieces-th of a block's share.  The pieces are laid
+    // pieces of at most a 2 split-th (the knob: a sixth) of a block's share.  The pieces are laid
     // out piece by piece and, within one, tile by tile, and dealt to the blocks
     // in this order (schedule_list): the tiles of a sector then run side by
     // side over the same items, and their operands, read by one row and one
     // column of tiles each, come from L2 (24 orbitals, M=500: phase 2 read
     // 2.4 GB of its 2.6 GB from memory before).  Sectors with more work first.
-    constexpr double kPieces = 6.0;
     std::vector<double> sec_cost(nsec, 0.0), sec_tile(nsec, 0.0);
     double stream_total = 0.0;
     for (int s = 0; s < nsec; ++s) {
@@ -1800,7 +1800,7 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
       stream_total += sec_cost[s];
     }
     const int nblk = (plan.tcx ? tcx_blocks_per_sm() : tc_blocks_per_sm(nb)) * nsm;
-    const double piece = seq ? 1e300 : std::max(stream_total / (kPieces * nblk), 12000.0);
+    const double piece = seq ? 1e300 : std::max(stream_total / (2.0 * kn.split * nblk), 12000.0);
     std::vector<int> sec_order(nsec);
     for (int s = 0; s < nsec; ++s) sec_order[s] = s;
     if (!seq)

@@ -58,16 +58,16 @@ struct DevArray {
 // Knobs of the tensor-core work-list schedule (the tile shapes follow the
 // sectors: 128-row A tiles and up to 64-column B tiles, cut to each sector).
 struct TcKnobs {
-  double item_cost = 400.0;  // LPT cost of an item on top of its K x N work
-  double split = 3.0;        // phase-2 pieces per persistent block (tile splitting)
+  double item_cost = 400.0;  // cost of an item on top of its K x N work
+  double split = 3.0;        // half the phase-2 pieces per persistent block (tile splitting)
   int group = 16;            // items per tensor-core accumulation group
   int per_sector = 0;        // 1: one launch per sector, one block per task (baseline)
   int nb = 64;               // output-tile width: 64 (two pipelines per SM) or 128 (one, wider MMAs)
-  // task order across the persistent blocks: 0 longest-processing-time
-  // assignment (column tiles of a row kept on one block), 1 waves (task
-  // order cut into waves of one task per block, balanced within each wave,
-  // so that the blocks work on neighbouring tiles of a sector together and
-  // share its operand tiles in L2)
+  // tasks across the persistent blocks: 0 phase 1 by longest processing time
+  // (column tiles of a row kept on one block), phase 2 in order, each task to
+  // the block that is free first, so that the blocks work on neighbouring tiles
+  // of a sector together and share its operand tiles in L2; 1 both in waves
+  // (task order cut into waves of one task per block, balanced within each)
   int waves = 0;
   bool operator==(const TcKnobs& o) const {
     return item_cost == o.item_cost && split == o.split && group == o.group && per_sector == o.per_sector &&

@@ -102,3 +102,27 @@ def test_exact_far_scales(gpu_ctx, ea, eb, ep):
         assert np.linalg.norm((got - ref) / big) <= 1e-11 * np.linalg.norm(ref / big)
     finally:
         gpu_ctx.set_precision("fp64")
+
+
+def test_split_knob_sets_the_pieces(gpu_ctx, monkeypatch):
+    """The split knob cuts the phase-2 tiles into more pieces, for the same
+    product (a sector of 12 x 12 or more tiles, each above a piece's least)."""
+    rng = np.random.default_rng(12)
+    tasks = []
+    try:
+        gpu_ctx.set_precision("bf16x3tc")
+        sb, sigma = superblock(gpu_ctx, 1500, 1500, rng, 40)
+        psi = rng.standard_normal((1500, 1500))
+        ref = sigma(psi)
+        for split in ("1", "3", "6"):
+            monkeypatch.setenv("BGPU_TC_SPLIT", split)
+            gpu_ctx.set_tc_stacking(64 if split == "3" else 56)  # (another limit: the plan is made again)
+            got = gpu_ctx.sigma(sb, psi.reshape(-1)).reshape(1500, 1500)
+            assert np.linalg.norm(got - ref) <= 2e-5 * np.linalg.norm(ref)
+            info = gpu_ctx.superblock_info(sb)
+            assert info["tc_split"] == float(split)
+            tasks.append(info["tc_phase2_tasks"])
+    finally:
+        gpu_ctx.set_tc_stacking(64)
+        gpu_ctx.set_precision("fp64")
+    assert tasks[0] < tasks[1] < tasks[2], tasks
