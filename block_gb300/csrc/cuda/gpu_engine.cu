@@ -2045,8 +2045,6 @@ void GpuEngine::schedule_tc(const Superblock& sb, SigmaPlan& plan, const TcKnobs
           x.b_base = (int64_t)(plan.tc_pool[it.b_pool] + it.b_off + 2 * (int64_t)nb * T.tn * it.kp);
           x.kp = it.kp;
           x.alpha = it.alpha;
-          x.a_pool = it.a_pool;
-          x.b_pool = it.b_pool;
           uint32_t f = f0 | (i == T.ibeg ? kTcFirst : 0) | (i + 1 == T.iend ? kTcLast : 0);
           const bool foldable = phase == 2 && it.alpha == 1.0f;
           if (gn == 0) f |= kTcGStart;

@@ -112,8 +112,8 @@ struct TcTile {
 
 // One item as the persistent kernel streams it (64 bytes): the items of a
 // block's tasks, flattened in processing order, each carrying what the
-// producer, MMA and epilogue roles need, so that a warp loads 32 of them
-// with one coalesced access and no role chases task -> item pointers.
+// producer, MMA and epilogue roles need, so that no role chases task -> item
+// pointers; each role reads its part of the next records ahead.
 //   a_base / b_base: device addresses of the row tile (128 rows of A, NB of B)
 //     in their pools
 //   out_base: phase 1: S row-tile base (pool S); phase 2 direct: sigma
@@ -138,8 +138,8 @@ struct __align__(16) TcWork {
   float alpha;
   int16_t h_a, h_b, valid_rows, valid_cols;
   int32_t out_ld, col0;
-  uint8_t a_pool, b_pool, flags, pad;
-  int32_t pad2[3];
+  uint8_t pad[2], flags, pad2;
+  int32_t pad3[3];
 };
 static_assert(sizeof(TcWork) == 64, "TcWork is 64 bytes");
 
