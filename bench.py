@@ -190,16 +190,6 @@ def fp64_peak_tflops():
         return None
 
 
-# DRAM bytes (read + write) of the two tensor-core sigma kernels per product,
-# from ncu captures of this bench's workloads (profiles/tc_sigma_*.md), made
-# before the stage-1 products of small blocks were stacked (at M=2000 the
-# stacks replace 37 % of the phase-1 tiles, all of small blocks; the
-# operands they read are the same bytes)
-NCU_TRAFFIC = {("tests/golden/syn24/dmrg.conf", 11, "bf16x3tc"): 3.275e9,
-               ("tests/golden/syn30/dmrg.conf", 14, "bf16x3tc"): 244.19e9}
-NCU_TRAFFIC_NOTE = "ncu capture before stacked stage-1 tiles (profiles/tc_sigma_bf16x3tc_syn30_m2000.md)"
-
-
 def measured_peaks():
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
@@ -267,23 +257,12 @@ def config_dict(conf, partition, n, prec, arena_mb):
 
 
 def run_reference(a):
-    rank, world, _ = dist_env()
-    if rank != 0:
-        return
-    threads = os.cpu_count() or 1
-    r = cpu_sample(a.conf, a.partition, max(1, min(a.steps, 2)))
-    v = r["flops"] / r["seconds"] / 1e12
-    sample = ("%d sigma product(s) on a superblock with the benchmark's sectors, operator catalogue and pair list "
-              "and seeded random operator values (CPU oracle, OpenMP over operator pairs, per-thread sigma copies)"
-              % max(1, min(a.steps, 2)))
-    line = {"impl": "reference", "metric": METRIC, "value": v, "unit": "TFLOP/s", "n_gpus": a.gpus,
-            "steps": a.steps, "warmup": a.warmup, "ms_per_step": r["seconds"] * 1e3, "higher_is_better": True,
-            "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
-            "config": config_dict(a.conf, a.partition, r["psi"], "fp64", 8.0 * r["arena"] / 1e6),
-            "cpu_baseline": {"value": v, "unit": "TFLOP/s", "cores": r["threads"] or threads, "kind": "port",
-                             "sample": sample, "dgemm": r["dgemm"]},
-            "e2e": {"value": v, "unit": "TFLOP/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
-    print(json.dumps(line), flush=True)
+    rank, _, _ = dist_env()
+    if rank == 0:
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "not a Python package, and its C++ build needs Boost, BLAS/LAPACK and "
+                                         "gfortran, which are not installed (the CPU oracle's sigma is cpu_baseline)"}),
+              flush=True)
 
 
 def sweep_entry(ctx, conf, st, seconds, e):
@@ -384,11 +363,8 @@ def run_ours(a):
         kname = ("tc_sigma_kernel<1>+<2> (tcgen05/TMEM two-phase sector GEMMs, bf16 slices)" if tc_path else
                  "tcx_sigma_kernel<1>+<2> (tcgen05/TMEM exact-slice sector GEMMs, 6 bf16 digits, FP64 sums)"
                  if a.precision == "exacttc" else "fused_sigma_kernel (two-stage sector GEMMs, bf16 slices)")
-        traffic = NCU_TRAFFIC.get((os.path.relpath(a.conf, ROOT), a.partition, a.precision))
         roof = {"bound": "tensor", "achieved": achieved, "peak": pk, "unit": "TFLOP/s", "frac": achieved / pk,
-                "traffic": traffic, "traffic_unit": "bytes per sigma (both tensor-core kernels, ncu)",
-                "traffic_source": NCU_TRAFFIC_NOTE if traffic else None,
-                "hbm_time_of_traffic_ms": (traffic / (peaks.get("hbm_gbs", 6800.0) * 1e9) * 1e3) if traffic else None,
+                "traffic": None,
                 "kernel": kname,
                 "peak_source": ("bf16_tflops of measured" if peaks else "fallback 1900"),
                 "products_per_logical_product": prods,
