@@ -403,13 +403,6 @@ struct PlanTimer {
   ~PlanTimer() { acc += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count(); }
 };
 
-// Longest-processing-time assignment of tasks to `nblocks` persistent
-// blocks; block j runs order[ranges[j].x .. ranges[j].y), in task order.
-// Tasks with the same bundle id (contiguous in task order; for instance the
-// column tiles of one row of an output sector, which read the same A
-// operands) stay together on one block, consecutive, unless a bundle costs
-// more than a block's fair share, in which case it is cut into pieces of at
-// most that share.
 // Clocks of an exact item on its block: of each quarter of 32 TMEM lanes that
 // its rows take (read-out and sums), and of K times columns (MMAs).  Fitted to
 // the blocks' clocks at 20 orbitals M=300 (0.7 % rms in phase 1, 4 % in phase 2);
@@ -456,6 +449,13 @@ void interleave_tasks(const std::vector<int>& rows, const std::vector<int>& coun
   }
 }
 
+// Longest-processing-time assignment of tasks to `nblocks` persistent
+// blocks; block j runs order[ranges[j].x .. ranges[j].y), in task order.
+// Tasks with the same bundle id (contiguous in task order; for instance the
+// column tiles of one row of an output sector, which read the same A
+// operands) stay together on one block, consecutive, unless a bundle costs
+// more than a block's fair share, in which case it is cut into pieces of at
+// most that share.
 void schedule_lpt(const std::vector<double>& cost, const std::vector<int64_t>& bundle, int nblocks,
                   std::vector<int>& order, std::vector<int2>& ranges) {
   const int n = (int)cost.size();

@@ -340,14 +340,17 @@ __device__ __forceinline__ EpiRec load_epi(const TcWork* __restrict__ w, int i, 
 // accumulators rotate between groups.  Operand pieces are streamed by bulk
 // copies through the shared-memory ring.  Persistent: block j walks the work
 // records [ranges[j].x, ranges[j].y), and the pipeline runs across task
-// boundaries; the producer and the MMA issuer are one thread each.
+// boundaries; one lane produces, one warp issues the MMAs.
 // The epilogue folds each group sum into a compensated (hi, lo) f32 pair per
-// element.  Most groups of a phase-2 task are single items (a stage-1 product
-// read by several spin couplings keeps its factor), so that the fold, not the
-// MMAs, bounded phase 2: with the pairs in TMEM and four warps it took about
-// 3500 clocks a 128 x 128 item (24 orbitals, M=500: 331 items an SM, 680 us).
-// The pairs now stay in registers, 64 columns a thread, folded two values an
-// instruction.
+// element, 64 columns a thread, two values an instruction (168 registers a
+// thread, 68 bytes of them spilled).  With the pairs in TMEM and four warps
+// phase 2 took 680 us at 24 orbitals, M=500; 441 now.
+// Bound, of the issuer's clocks in phase 2: 24 orbitals M=500 (spin 0: all
+// factors are 1, nine items a group) MMAs 48 %, waits for operand pieces 36 %,
+// for an accumulator 11 %; 18 orbitals M=1000 65, 28 and 9 %.  Targets with
+// spin: a stage-1 product read by several couplings keeps its factor and is a
+// group by itself (triplet M=101: waits for an accumulator, that is the folds,
+// 48 %, MMAs 15 %).
 template <int PHASE, int NB>
 __global__ void __launch_bounds__(TcCfg<NB>::kThreads, TcCfg<NB>::kBlocksPerSm)
     tc_sigma_kernel(TcBufs b, const TcWork* __restrict__ work, const int2* __restrict__ ranges,

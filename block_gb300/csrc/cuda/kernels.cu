@@ -28,7 +28,7 @@ namespace dev {
 // short K nor a barrier per item are paid; the items' descriptors are staged
 // 16 at a time.  Seven blocks share an SM and hide each other's loads.
 // Measured, sigma of 16 orbitals at M=150 (sectors of up to 101 states,
-// 2.24 GFLOP): 7.3 -> 2.6 ms, 0.85 of 1.1 TFLOP/s, against 64 x 64 tiles of
+// 2.24 GFLOP): 7.3 -> 2.6 ms, 0.85 of the pipe's 1.26 TFLOP/s, against 64 x 64 tiles of
 // 4 x 4 outputs a thread and slabs of 16 K padded with zeros.
 // ------------------------------------------------------------------------
 namespace {

@@ -116,8 +116,8 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
 }
 
 // The same in code that a whole warp runs, carried out by the lane with `on`
-// set.  The operands then stay in uniform registers; in code that one lane
-// runs by itself the compiler moves each of them there before every MMA.
+// set (24 orbitals M=500, with the sums of phase 2 in registers and its pieces
+// side by side: 1005 -> 801 us a product).
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile(
