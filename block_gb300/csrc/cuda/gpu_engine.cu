@@ -62,12 +62,12 @@ std::mutex g_stage_mu;
 std::map<cudaStream_t, StageRing> g_stage;
 }  // namespace
 
-cudaError_t stage_h2d(void* dst, const void* src, size_t bytes, cudaStream_t s) {
-  if (bytes == 0) return cudaSuccess;
-  // block arenas (restarts) are copied directly: a ring for them would pin
-  // several times their size
-  constexpr size_t kStageMax = size_t(256) << 20;
-  if (bytes > kStageMax) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
+namespace {
+// `bytes` to dst through the ring, written there by fill; *staged is false, and
+// nothing was copied, where there is no memory for the ring
+template <class Fill>
+cudaError_t stage_with(void* dst, size_t bytes, cudaStream_t s, bool* staged, Fill fill) {
+  *staged = true;
   std::lock_guard<std::mutex> lk(g_stage_mu);
   StageRing& st = g_stage[s];
   const size_t need = (bytes + 255) & ~(size_t)255;
@@ -81,7 +81,8 @@ cudaError_t stage_h2d(void* dst, const void* src, size_t bytes, cudaStream_t s) 
       cudaGetLastError();
       st.ring = nullptr;
       st.cap = 0;
-      return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);  // unstaged
+      *staged = false;
+      return cudaSuccess;
     }
   }
   size_t p = st.head;
@@ -99,7 +100,7 @@ cudaError_t stage_h2d(void* dst, const void* src, size_t bytes, cudaStream_t s) 
       st.inflight.pop_front();
     }
   }
-  std::memcpy(st.ring + p, src, bytes);
+  fill(st.ring + p);
   cudaError_t e = cudaMemcpyAsync(dst, st.ring + p, bytes, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return e;
   cudaEvent_t ev;
@@ -113,6 +114,38 @@ cudaError_t stage_h2d(void* dst, const void* src, size_t bytes, cudaStream_t s) 
   st.inflight.push_back({p, p + need, ev});
   st.head = p + need;
   return cudaSuccess;
+}
+}  // namespace
+
+cudaError_t stage_h2d(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+  if (bytes == 0) return cudaSuccess;
+  // block arenas (restarts) are copied directly: a ring for them would pin
+  // several times their size
+  constexpr size_t kStageMax = size_t(256) << 20;
+  bool staged = false;
+  if (bytes <= kStageMax) {
+    const cudaError_t e = stage_with(dst, bytes, s, &staged, [&](char* to) { std::memcpy(to, src, bytes); });
+    if (e != cudaSuccess || staged) return e;
+  }
+  return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
+}
+
+void DevLists::upload(DevArray<char>& memory, cudaStream_t s) {
+  memory.release(s);
+  if (total == 0) return;
+  cuda_check(cudaMallocAsync((void**)&memory.d, total, s), "cudaMallocAsync(lists)");
+  memory.n = total;
+  for (const Part& p : parts) *p.at = memory.d + p.off;
+  // one copy of all, unless the ring, four times the largest copy, would grow by it
+  bool staged = false;
+  if (total <= (size_t(16) << 20))
+    cuda_check(stage_with(memory.d, total, s, &staged,
+                          [&](char* to) {
+                            for (const Part& p : parts) std::memcpy(to + p.off, p.src, p.bytes);
+                          }),
+               "upload lists");
+  if (!staged)
+    for (const Part& p : parts) cuda_check(stage_h2d(memory.d + p.off, p.src, p.bytes, s), "upload list");
 }
 
 void release_staging(cudaStream_t s) {
@@ -135,9 +168,10 @@ void DevArray<T>::upload(const std::vector<T>& h, cudaStream_t s) {
 }
 template <class T>
 void DevArray<T>::release(cudaStream_t s) {
-  if (d) cudaFreeAsync(d, s);
+  if (d && !view) cudaFreeAsync(d, s);
   d = nullptr;
   n = 0;
+  view = false;
 }
 
 GpuEngine::GpuEngine(int device) : device_(device) {
@@ -567,9 +601,17 @@ void schedule_list(const std::vector<double>& cost, int nblocks, std::vector<int
   }
 }
 
+size_t tile_count(int m, int n, int tile = dev::kGemmTile) {
+  return (size_t)((m + tile - 1) / tile) * ((n + tile - 1) / tile);
+}
 void add_tasks(std::vector<dev::GemmTask>& t, int unit, int m, int n, int tile = dev::kGemmTile) {
-  for (int a = 0; a < (m + tile - 1) / tile; ++a)
-    for (int b = 0; b < (n + tile - 1) / tile; ++b) t.push_back({unit, a, b});
+  const int na = (m + tile - 1) / tile, nb = (n + tile - 1) / tile;
+  if (std::max(na, nb) > INT16_MAX) throw std::runtime_error("matrix of more than 2^15 tiles");
+  const size_t at = t.size();
+  t.resize(at + (size_t)na * nb);
+  dev::GemmTask* p = t.data() + at;
+  for (int a = 0; a < na; ++a)
+    for (int b = 0; b < nb; ++b) *p++ = {unit, a, b};
 }
 }  // namespace
 
@@ -704,6 +746,21 @@ void GpuEngine::build_block(Block& big, const Block& a, const Block& b,
 
 // ------------------------------------------------------------------ sigma
 
+void PlanLists::clear(size_t nsec) {
+  auto bytes = [](const auto& v) { return v.capacity() * sizeof(v[0]); };
+  size_t held = bytes(u1) + bytes(u2) + bytes(i1) + bytes(i2) + bytes(t1) + bytes(t2) + bytes(per_sector);
+  for (const auto& v : per_sector) held += bytes(v);
+  if (held > kKeep) *this = PlanLists{};
+  u1.clear();
+  u2.clear();
+  i1.clear();
+  i2.clear();
+  t1.clear();
+  t2.clear();
+  for (auto& v : per_sector) v.clear();
+  if (per_sector.size() < nsec) per_sector.resize(nsec);
+}
+
 // Compiles TensorMultiply (operatorfunctions.C:485-537) over all operator
 // pairs of SpinBlock::multiplyH into two grouped-GEMM launches:
 //   stage 1: M[t,lQ,lQ',rQ'] = s_L * A(lQ,lQ') * psi(lQ',rQ')
@@ -718,9 +775,9 @@ void GpuEngine::plan_sigma(const Superblock& sb, SigmaPlan& plan) {
   const int J = sb.target.s2;
   const auto by_l = sectors_by_left(sb);
   // buffers: 0 = L arena, 1 = R arena, 2 = psi, 3 = sigma, 4 = scratch
-  std::vector<dev::GemmUnit> u1;
-  std::vector<dev::GemmItem> i1;
-  std::vector<std::vector<dev::GemmItem>> per_sector(sb.sectors.size());
+  plan_lists_.clear(sb.sectors.size());
+  PlanLists lists = std::move(plan_lists_);
+  auto& [u1, u2, i1, i2, per_sector, t1, t2] = lists;
   int64_t scratch = 0;
   double flops = 0.0, bytes = 0.0;
   std::set<std::pair<int, OpKey>> used;
@@ -815,9 +872,6 @@ void GpuEngine::plan_sigma(const Superblock& sb, SigmaPlan& plan) {
   // fair share of the FP64 pipe's work is split along its item list into
   // units writing partial sectors after the stage-1 intermediates, summed
   // into sigma in a fixed order by the build-copy kernel
-  std::vector<dev::GemmUnit> u2;
-  std::vector<dev::GemmItem> i2;
-  std::vector<dev::GemmTask> t1, t2;
   std::vector<dev::CopyUnit> ru;
   std::vector<dev::CopyItem> ri;
   // Work of a tile's share of a sector, in clocks of one SM: its FMAs at two
@@ -828,18 +882,20 @@ void GpuEngine::plan_sigma(const Superblock& sb, SigmaPlan& plan) {
   // and not 2.6; the former rule, a quarter of an SM's share and at least
   // 4096 K, left the 20 sectors of 12 orbitals, M=50 to 20 blocks: 7.1 ms
   // for the whole product, now 0.19).
-  auto tiles_of = [](const Superblock::Sector& S) {
-    return (double)((S.rows + dev::kGemmTile - 1) / dev::kGemmTile) * ((S.cols + dev::kGemmTile - 1) / dev::kGemmTile);
-  };
-  auto item_cost = [&](const Superblock::Sector& S, const dev::GemmItem& g) {
-    return 0.5 * S.rows * S.cols * g.k / tiles_of(S) + 150.0;
-  };
-  std::vector<double> tile_cost(sb.sectors.size(), 0.0);
+  auto tiles_of = [](const Superblock::Sector& S) { return (double)tile_count(S.rows, S.cols); };
+  std::vector<double> tile_cost(sb.sectors.size(), 0.0), k_cost(sb.sectors.size());
   double total_cost = 0.0;
+  size_t n_items = 0;
   for (size_t s = 0; s < sb.sectors.size(); ++s) {
-    for (auto& g : per_sector[s]) tile_cost[s] += item_cost(sb.sectors[s], g);
-    total_cost += tile_cost[s] * tiles_of(sb.sectors[s]);
+    const auto& S = sb.sectors[s];
+    int64_t k = 0;
+    for (auto& g : per_sector[s]) k += g.k;
+    k_cost[s] = 0.5 * S.rows * S.cols / tiles_of(S);
+    tile_cost[s] = k_cost[s] * k + 150.0 * per_sector[s].size();
+    total_cost += tile_cost[s] * tiles_of(S);
+    n_items += per_sector[s].size();
   }
+  i2.reserve(n_items);
   double share = std::max(total_cost / (32.0 * sm_count()), 1500.0);
   auto chunks_of = [&](size_t s) {
     return std::max(1, std::min((int)per_sector[s].size(), (int)std::ceil(tile_cost[s] / share)));
@@ -856,6 +912,13 @@ void GpuEngine::plan_sigma(const Superblock& sb, SigmaPlan& plan) {
       if (extra == 0 || scratch + extra <= (int64_t)BGPU_NOALLOC_SCRATCH_DOUBLES) break;
     }
   int64_t partial = scratch;  // partial sectors follow the stage-1 intermediates
+  std::vector<uint64_t> heavier;  // falling clocks of the units' tiles, then the units
+  size_t n_tasks = 0;
+  auto unit_done = [&](const dev::GemmUnit& u, double c) {
+    heavier.push_back((uint64_t)(UINT32_MAX - (uint32_t)std::min(c, 4e9)) << 32 | u2.size());
+    n_tasks += tile_count(u.m, u.n);
+    u2.push_back(u);
+  };
   for (size_t s = 0; s < sb.sectors.size(); ++s) {
     const auto& S = sb.sectors[s];
     const auto& items = per_sector[s];
@@ -869,9 +932,9 @@ void GpuEngine::plan_sigma(const Superblock& sb, SigmaPlan& plan) {
       u.n = S.cols;
       u.beta_one = 0;
       u.ibeg = (int)i2.size();
-      for (auto& g : items) i2.push_back(g);
+      i2.insert(i2.end(), items.begin(), items.end());
       u.iend = (int)i2.size();
-      u2.push_back(u);
+      unit_done(u, tile_cost[s]);
       continue;
     }
     dev::CopyUnit cu{};
@@ -885,7 +948,8 @@ void GpuEngine::plan_sigma(const Superblock& sb, SigmaPlan& plan) {
     for (int c = 0; c < nchunks && a < items.size(); ++c) {
       size_t e = a;
       double acc = 0.0;
-      while (e < items.size() && (acc < per || e == a || c == nchunks - 1)) acc += item_cost(S, items[e++]);
+      while (e < items.size() && (acc < per || e == a || c == nchunks - 1))
+        acc += k_cost[s] * items[e++].k + 150.0;
       dev::GemmUnit u{};
       u.c_buf = 4;
       u.c_off = partial;
@@ -894,9 +958,9 @@ void GpuEngine::plan_sigma(const Superblock& sb, SigmaPlan& plan) {
       u.n = S.cols;
       u.beta_one = 0;
       u.ibeg = (int)i2.size();
-      for (size_t x = a; x < e; ++x) i2.push_back(items[x]);
+      i2.insert(i2.end(), items.begin() + a, items.begin() + e);
       u.iend = (int)i2.size();
-      u2.push_back(u);
+      unit_done(u, acc);
       dev::CopyItem ci{};
       ci.s_off = partial;
       ci.lds = S.cols;
@@ -910,27 +974,15 @@ void GpuEngine::plan_sigma(const Superblock& sb, SigmaPlan& plan) {
     ru.push_back(cu);
   }
   scratch = partial;
+  size_t n1 = 0;
+  for (const auto& u : u1) n1 += tile_count(u.m, u.n);
+  t1.reserve(n1);
   for (int u = 0; u < (int)u1.size(); ++u) add_tasks(t1, u, u1[u].m, u1[u].n);
   // heavier output tiles first
-  std::vector<std::pair<double, int>> cost;
-  for (int u = 0; u < (int)u2.size(); ++u) {
-    double c = 0;
-    const int nth = (u2[u].m + dev::kGemmTile - 1) / dev::kGemmTile, ntw = (u2[u].n + dev::kGemmTile - 1) / dev::kGemmTile;
-    const double area = (double)u2[u].m * u2[u].n / (nth * ntw);
-    for (int i = u2[u].ibeg; i < u2[u].iend; ++i) c += 0.5 * area * i2[i].k + 150.0;
-    cost.push_back({-c, u});
-  }
-  std::stable_sort(cost.begin(), cost.end());
-  for (auto& c : cost) add_tasks(t2, c.second, u2[c.second].m, u2[c.second].n);
+  std::sort(heavier.begin(), heavier.end());
+  t2.reserve(n_tasks);
+  for (const uint64_t h : heavier) add_tasks(t2, (int)(uint32_t)h, u2[(uint32_t)h].m, u2[(uint32_t)h].n);
   laps.lap("stage-2 units");
-  plan.u1.upload(u1, stream_);
-  plan.i1.upload(i1, stream_);
-  plan.t1.upload(t1, stream_);
-  plan.u2.upload(u2, stream_);
-  plan.i2.upload(i2, stream_);
-  plan.t2.upload(t2, stream_);
-  plan.ru.upload(ru, stream_);
-  plan.ri.upload(ri, stream_);
   plan.scratch_elems = scratch;
   plan.scratch = nullptr;  // allocated by the first FP64 product
   plan.flops = flops;
@@ -940,7 +992,6 @@ void GpuEngine::plan_sigma(const Superblock& sb, SigmaPlan& plan) {
   plan.nstage1_units = (int)u1.size();
   plan.nstage2_units = (int)u2.size();
   plan.nitems = (int)(i1.size() + i2.size());
-  laps.lap("uploads");
   // diagonal work list (diagonalH, spinblock.C:855-899)
   std::vector<dev::DiagUnit> du;
   std::vector<dev::DiagItem> di;
@@ -975,9 +1026,21 @@ void GpuEngine::plan_sigma(const Superblock& sb, SigmaPlan& plan) {
   std::vector<dev::GemmTask> dtask;
   for (int u = 0; u < (int)du.size(); ++u) add_tasks(dtask, u, du[u].rows, du[u].cols, dev::kDiagTile);
   laps.lap("diagonal lists");
-  plan.du.upload(du, stream_);
-  plan.di.upload(di, stream_);
-  plan.dtask.upload(dtask, stream_);
+  DevLists up;
+  up.add(plan.u1, u1, stream_);
+  up.add(plan.i1, i1, stream_);
+  up.add(plan.t1, t1, stream_);
+  up.add(plan.u2, u2, stream_);
+  up.add(plan.i2, i2, stream_);
+  up.add(plan.t2, t2, stream_);
+  up.add(plan.ru, ru, stream_);
+  up.add(plan.ri, ri, stream_);
+  up.add(plan.du, du, stream_);
+  up.add(plan.di, di, stream_);
+  up.add(plan.dtask, dtask, stream_);
+  up.upload(plan.fp64_lists, stream_);
+  plan_lists_ = std::move(lists);
+  laps.lap("uploads");
 }
 
 void GpuEngine::free_tc(SigmaPlan& p) {
@@ -1047,6 +1110,7 @@ void GpuEngine::free_plan(SigmaPlan& p) {
   p.dtask.release(stream_);
   p.ru.release(stream_);
   p.ri.release(stream_);
+  p.fp64_lists.release(stream_);
   free(p.scratch);
   p.scratch = nullptr;
 }

@@ -51,8 +51,34 @@ template <class T>
 struct DevArray {
   T* d = nullptr;
   size_t n = 0;
+  bool view = false;  // lies in another array's memory (DevLists)
   void upload(const std::vector<T>& h, cudaStream_t s);
   void release(cudaStream_t s);
+};
+
+// Work lists that live and go together: one allocation, which `memory` owns and
+// the arrays view, and one staged copy (an allocation, a copy and an event for
+// each of a plan's eleven lists took a third of the time to define a small
+// superblock).
+struct DevLists {
+  struct Part {
+    const void* src;
+    size_t bytes, off;
+    char** at;
+  };
+  std::vector<Part> parts;
+  size_t total = 0;
+  template <class T>
+  void add(DevArray<T>& a, const std::vector<T>& h, cudaStream_t s) {
+    a.release(s);
+    if (h.empty()) return;
+    a.n = h.size();
+    a.view = true;
+    parts.push_back({h.data(), h.size() * sizeof(T), total, reinterpret_cast<char**>(&a.d)});
+    total += (parts.back().bytes + 255) & ~(size_t)255;
+  }
+  // the added vectors must still be there
+  void upload(DevArray<char>& memory, cudaStream_t s);
 };
 
 // Knobs of the tensor-core work-list schedule (the tile shapes follow the
@@ -76,8 +102,20 @@ struct TcKnobs {
 };
 struct TcHostPlan;  // item lists of a tensor-core plan, kept for rescheduling
 
+// Host side of the FP64 lists while a plan is made.  The engine keeps it from
+// plan to plan (a sweep makes one at every bond), up to kKeep bytes.
+struct PlanLists {
+  static constexpr size_t kKeep = size_t(64) << 20;
+  std::vector<dev::GemmUnit> u1, u2;
+  std::vector<dev::GemmItem> i1, i2;
+  std::vector<std::vector<dev::GemmItem>> per_sector;
+  std::vector<dev::GemmTask> t1, t2;
+  void clear(size_t nsec);  // empty, for nsec sectors
+};
+
 // Compiled sigma = H psi work lists of one superblock.
 struct SigmaPlan {
+  DevArray<char> fp64_lists;  // memory of the lists from here to ri
   DevArray<dev::GemmUnit> u1, u2;
   DevArray<dev::GemmItem> i1, i2;
   DevArray<dev::GemmTask> t1, t2;
@@ -365,6 +403,7 @@ class GpuEngine : public Engine {
   cudaEvent_t side_fork_ = nullptr, side_join_ = nullptr;
   // thread-block clusters of the eigensolver on this device, asked for once
   dev::EigClusters eig_clusters_{};
+  PlanLists plan_lists_;
   bool eig_clusters_known_ = false;
   // rotation that made each renormalised block (big-block quantum q: n[q] x m[q]
   // row-major at off[q]), kept for the wavefunction guess transform

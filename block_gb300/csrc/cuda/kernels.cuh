@@ -43,8 +43,11 @@ struct GemmUnit {
 
 struct GemmTask {
   int32_t unit;
-  int32_t tm, tn;  // tile indices
+  int16_t tm, tn;  // tile indices
+  GemmTask() {}    // (lists are resized, then written)
+  GemmTask(int u, int a, int b) : unit(u), tm((int16_t)a), tn((int16_t)b) {}
 };
+static_assert(sizeof(GemmTask) == 8, "lists of several 100 000");
 constexpr int kGemmTile = 32;  // largest output-tile edge of the grouped GEMM
 constexpr int kGemmTileSmall = 16;  // edge for lists that leave SMs idle with kGemmTile
 constexpr int kDiagTile = 64;  // and of the diagonal tiles
