@@ -746,11 +746,14 @@ void GpuEngine::build_block(Block& big, const Block& a, const Block& b,
 
 // ------------------------------------------------------------------ sigma
 
+size_t PlanLists::bytes() const {
+  auto of = [](const auto& v) { return v.capacity() * sizeof(v[0]); };
+  size_t n = of(u1) + of(u2) + of(i1) + of(i2) + of(t1) + of(t2) + of(per_sector);
+  for (const auto& v : per_sector) n += of(v);
+  return n;
+}
+
 void PlanLists::clear(size_t nsec) {
-  auto bytes = [](const auto& v) { return v.capacity() * sizeof(v[0]); };
-  size_t held = bytes(u1) + bytes(u2) + bytes(i1) + bytes(i2) + bytes(t1) + bytes(t2) + bytes(per_sector);
-  for (const auto& v : per_sector) held += bytes(v);
-  if (held > kKeep) *this = PlanLists{};
   u1.clear();
   u2.clear();
   i1.clear();
@@ -1039,7 +1042,7 @@ void GpuEngine::plan_sigma(const Superblock& sb, SigmaPlan& plan) {
   up.add(plan.di, di, stream_);
   up.add(plan.dtask, dtask, stream_);
   up.upload(plan.fp64_lists, stream_);
-  plan_lists_ = std::move(lists);
+  if (lists.bytes() <= PlanLists::kKeep) plan_lists_ = std::move(lists);
   laps.lap("uploads");
 }
 

@@ -103,7 +103,7 @@ struct TcKnobs {
 struct TcHostPlan;  // item lists of a tensor-core plan, kept for rescheduling
 
 // Host side of the FP64 lists while a plan is made.  The engine keeps it from
-// plan to plan (a sweep makes one at every bond), up to kKeep bytes.
+// plan to plan (a sweep makes one at every bond) unless it is above kKeep bytes.
 struct PlanLists {
   static constexpr size_t kKeep = size_t(64) << 20;
   std::vector<dev::GemmUnit> u1, u2;
@@ -111,6 +111,7 @@ struct PlanLists {
   std::vector<std::vector<dev::GemmItem>> per_sector;
   std::vector<dev::GemmTask> t1, t2;
   void clear(size_t nsec);  // empty, for nsec sectors
+  size_t bytes() const;
 };
 
 // Compiled sigma = H psi work lists of one superblock.
